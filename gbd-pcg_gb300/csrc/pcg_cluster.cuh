@@ -834,17 +834,142 @@ __device__ __forceinline__ void push_halo_tx(const T *dst_local, uint32_t to, co
     for (int q = 0; q < RPT; ++q) st_async(ra + (uint32_t)(q * sizeof(T)), v[q], rb);
 }
 
+// ---------------------------------------------------------------- reductions of
+// doubles.  GB300 issues FP64 at 2 lanes a clock per SM (64 times less than
+// FP32), so what bounds a reduction of doubles is the number of warp-wide FP64
+// instructions of the whole CTA, 16 clocks of the SM each, not its depth: a
+// butterfly in every warp is 5 W of them per value, the slot sums of every
+// thread up to 15 W, and a division or a comparison in every thread costs
+// again W times its chain.  Here the W warps only store their lanes' partials
+// (`wscr`, [value][warp][lane]); after a CTA barrier one warp per value adds
+// the W rows (W - 1 instructions) and finishes with one butterfly (5), sends
+// the CTA's sum to every CTA of the cluster as cluster_allreduce_tx does, adds
+// the C slots by a butterfly over the lanes, and evaluates the quotient and
+// the exit tests (`fin`), and a second CTA barrier hands the results to every
+// thread through shared memory.  Per iteration of the FP64 solver (3 values,
+// W = 8, C = 4) that is about 80 FP64 instructions a CTA instead of 450, beside
+// the 496 of its products.  In two halves like cluster_allreduce_tx; the first
+// half's barrier completes this CTA's stores made before the call.
+template <typename A>
+constexpr bool kOneWarpSums = std::is_same<A, double>::value;
+
+// What the summing warps hand to every thread, at the end of the slot array
+// (the slots of the last value in use end at C or, for C == 1, are not used).
+struct alignas(16) ReduceOut {
+    double sum[kMaxValues];
+    double ratio;                // a quotient of the kernel's type
+    uint32_t code[kMaxValues];   // exit tests, per value
+};
+static_assert(sizeof(ReduceOut) <= 64, "the last 8 doubles of the slot array");
+template <typename A>
+__device__ __forceinline__ ReduceOut *reduce_out(A *slots, uint32_t C) {
+    return reinterpret_cast<ReduceOut *>(slots + 2 * kMaxValues * slot_stride(C) - 64 / sizeof(A));
+}
+
+template <typename A, int NQ>
+__device__ __forceinline__ void onewarp_send(A (&v)[NQ], A *slots, A *wscr, int buf, TxReduce &tx, uint32_t C,
+                                             uint32_t rank, uint32_t extra_bytes) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) wscr[((uint32_t)q * nwarps + warp) * 32 + lane] = v[q];
+    __syncthreads();
+    if (C > 1 && threadIdx.x == 0)
+        mbar_arrive_expect_tx(tx.bar + buf, (uint32_t)(NQ * C * sizeof(A)) + extra_bytes);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if (warp != (uint32_t)q % nwarps) continue;
+        const A *x = wscr + (uint32_t)q * nwarps * 32 + lane;
+        A t[1] = {x[0]}, t1 = A(0);
+        uint32_t w = 1;
+#pragma unroll 4
+        for (; w + 1 < nwarps; w += 2) {
+            t[0] += x[w * 32];
+            t1 += x[w * 32 + 32];
+        }
+        if (w < nwarps) t[0] += x[w * 32];
+        if (nwarps > 2) t[0] += t1;
+        warp_sum_n<A, 1>(t);
+        v[q] = t[0];
+        if (C > 1 && lane < C) {
+            const uint32_t stride = (uint32_t)slot_stride(C);
+            A *sl = slots + ((size_t)buf * kMaxValues + q) * stride + rank;
+            st_async(map_rank_u32(smem_u32(sl), lane), t[0], map_rank_u32(smem_u32(tx.bar + buf), lane));
+        }
+    }
+}
+
+// `fin(q, sum, out)`: run by the lanes of the warp that summed value q, with
+// lane 0's stores to `out` kept (ratio, code[q]).
+template <typename A, int NQ, typename F>
+__device__ __forceinline__ const ReduceOut *onewarp_finish(A (&v)[NQ], A *slots, int buf, TxReduce &tx, uint32_t C,
+                                                           F &&fin) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    ReduceOut *out = reduce_out(slots, C);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if (warp != (uint32_t)q % nwarps) continue;
+        A s = v[q];
+        if (C > 1) {
+            mbar_wait_bounded(tx.bar + buf, (tx.parity >> buf) & 1u, tx.timed_out);
+            const A *sl = slots + ((size_t)buf * kMaxValues + q) * slot_stride(C);
+            s = lane < C ? sl[lane] : A(0);
+            for (uint32_t off = C > 8 ? 8 : (C > 4 ? 4 : (C > 2 ? 2 : 1)); off > 0; off >>= 1)
+                s += acc_shfl_xor(s, (int)off);
+            s = __shfl_sync(0xffffffffu, s, 0);
+        }
+        if (lane == 0) out->sum[q] = s;
+        fin(q, s, out);
+    }
+    if (C > 1) tx.parity ^= 1u << buf;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] = out->sum[q];
+    return out;
+}
+
 // A cluster-wide reduction of the cluster solver: the transaction-counted
 // form for C >= 2 (with `extra_bytes` of halo values expected on the same
-// buffer), the CTA-barrier form for C == 1.
+// buffer), the CTA-barrier form for C == 1; doubles by one warp per value.
 template <typename A, int NQ>
 __device__ __forceinline__ void solver_allreduce(A (&v)[NQ], A *slots, A *wscr, int buf, TxReduce &tx,
                                                  const cg::cluster_group &cluster, uint32_t C, uint32_t rank,
                                                  uint32_t extra_bytes) {
-    if (C == 1)
+    if constexpr (kOneWarpSums<A>) {
+        onewarp_send<A, NQ>(v, slots, wscr, buf, tx, C, rank, extra_bytes);
+        onewarp_finish<A, NQ>(v, slots, buf, tx, C, [](int, A, ReduceOut *) {});
+    } else if (C == 1)
         cluster_allreduce<A, NQ>(v, slots, wscr, buf, cluster, C, rank);
     else
         cluster_allreduce_tx<A, NQ>(v, slots, wscr, buf, tx, C, rank, extra_bytes);
+}
+
+// Exit tests of one iteration, as the summing warps report them.
+enum : uint32_t { kNotFinite = 1u, kExitTest = 2u };
+
+// The two reductions of an iteration with their quotient, for doubles: `pap`
+// and alpha = eta / pap (0 where pap is 0); r.z, r.r, beta = r.z / eta and the
+// exit tests (bits of kNotFinite and kExitTest).
+template <typename T, typename A>
+__device__ __forceinline__ T onewarp_alpha(A pap, const A &eta, ReduceOut *out, uint32_t lane) {
+    const T a = (pap == A(0)) ? T(0) : acc_ratio<T>(eta, pap);
+    if (lane == 0) {
+        *reinterpret_cast<T *>(&out->ratio) = a;
+        out->code[0] = acc_finite(pap) ? 0u : kNotFinite;
+    }
+    return a;
+}
+template <typename T, typename A>
+__device__ __forceinline__ void onewarp_beta(int q, A s, const A &eta, const A &tol, const A &thr, ReduceOut *out,
+                                             uint32_t lane) {
+    if (q == 0) {
+        const T b = acc_ratio<T>(s, eta);
+        if (lane == 0) {
+            *reinterpret_cast<T *>(&out->ratio) = b;
+            out->code[0] = (acc_finite(s) ? 0u : kNotFinite) | (acc_abs(s) < tol ? kExitTest : 0u);
+        }
+    } else if (lane == 0) {
+        out->code[1] = s <= thr ? kExitTest : 0u;
+    }
 }
 
 // The output fields of work item `item`'s descriptor, read again from memory
@@ -1272,14 +1397,25 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                     if (last_knot) push_halo_tx<T, RPT>(uh + i, rank + 1, y, tx, 0);
                 }
                 A pap;
+                uint32_t code1 = 0;
+                T alpha;
                 {
                     A v1[1] = {A(0)};
 #pragma unroll
                     for (int q = 0; q < RPT; ++q) acc_madd(v1[0], p[q], y[q]);
-                    solver_allreduce<A, 1>(v1, slots, wscr, 0, tx, cluster, C, rank, PTRI ? halo_in : 0u);
-                    pap = v1[0];
+                    if constexpr (kOneWarpSums<A>) {
+                        onewarp_send<A, 1>(v1, slots, wscr, 0, tx, C, rank, PTRI ? halo_in : 0u);
+                        const ReduceOut *o = onewarp_finish<A, 1>(
+                            v1, slots, 0, tx, C, [&](int, A s, ReduceOut *out) { onewarp_alpha<T>(s, eta, out, tid & 31); });
+                        alpha = *reinterpret_cast<const T *>(&o->ratio);
+                        code1 = o->code[0];
+                        pap = v1[0];
+                    } else {
+                        solver_allreduce<A, 1>(v1, slots, wscr, 0, tx, cluster, C, rank, PTRI ? halo_in : 0u);
+                        pap = v1[0];
+                        alpha = (pap == A(0)) ? T(0) : acc_ratio<T>(eta, pap);
+                    }
                 }
-                const T alpha = (pap == A(0)) ? T(0) : acc_ratio<T>(eta, pap);
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) {
                     lam[q] = fma_rn(alpha, p[q], lam[q]);
@@ -1310,7 +1446,8 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                 // are all in the window), the rest after the wait.  Either
                 // way, before the exit test, so that its loads and FMAs
                 // interleave with the slot sums.
-                T w[RPT];
+                T w[RPT], beta_h = T(0);
+                uint32_t code2 = 0;
                 {
                     A v2[2] = {A(0), A(0)};
 #pragma unroll
@@ -1318,7 +1455,19 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                         acc_madd(v2[0], r[q], z[q]);
                         if (relres) acc_madd(v2[1], r[q], r[q]);
                     }
-                    if (C > 1) {
+                    if constexpr (kOneWarpSums<A>) {
+                        // the first half's CTA barrier completes this CTA's z rows in the window
+                        onewarp_send<A, 2>(v2, slots, wscr, 1, tx, C, rank, halo_in);
+                        const bool halo_rows = C > 1 && __any_sync(0xffffffffu, first_knot || last_knot);
+                        if (!halo_rows) matS_rows(w);
+                        const ReduceOut *o = onewarp_finish<A, 2>(
+                            v2, slots, 1, tx, C,
+                            [&](int q, A s, ReduceOut *out) { onewarp_beta<T>(q, s, eta, tol, thr, out, tid & 31); });
+                        beta_h = *reinterpret_cast<const T *>(&o->ratio);
+                        code1 |= o->code[0] & kNotFinite;
+                        code2 = o->code[relres ? 1 : 0];
+                        if (halo_rows) matS_rows(w);
+                    } else if (C > 1) {
                         // its CTA barrier also completes this CTA's z rows in the window
                         cluster_allreduce_tx_send<A, 2>(v2, slots, wscr, 1, tx, C, rank, halo_in);
                         const bool halo_rows = __any_sync(0xffffffffu, first_knot || last_knot);
@@ -1333,9 +1482,16 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                     rr = v2[1];
                 }
                 ++iter;
-                if (!acc_finite(eta_new) || !acc_finite(pap)) { status = ST_BREAKDOWN; break; }
-                if (relres ? (rr <= thr) : (acc_abs(eta_new) < tol)) { status = ST_CONVERGED; break; }
-                const T beta = acc_ratio<T>(eta_new, eta);
+                T beta;
+                if constexpr (kOneWarpSums<A>) {
+                    if (code1 & kNotFinite) { status = ST_BREAKDOWN; break; }
+                    if (code2 & kExitTest) { status = ST_CONVERGED; break; }
+                    beta = beta_h;
+                } else {
+                    if (!acc_finite(eta_new) || !acc_finite(pap)) { status = ST_BREAKDOWN; break; }
+                    if (relres ? (rr <= thr) : (acc_abs(eta_new) < tol)) { status = ST_CONVERGED; break; }
+                    beta = acc_ratio<T>(eta_new, eta);
+                }
                 eta = eta_new;
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) {
@@ -1351,14 +1507,25 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                     if (last_knot) push_halo_tx<T, RPT>(uh + i, rank + 1, y, tx, 0);
                 }
                 A pap;
+                uint32_t code1 = 0;
+                T alpha;
                 {
                     A v1[1] = {A(0)};
 #pragma unroll
                     for (int q = 0; q < RPT; ++q) acc_madd(v1[0], p[q], y[q]);
-                    solver_allreduce<A, 1>(v1, slots, wscr, 0, tx, cluster, C, rank, PTRI ? halo_in : 0u);
-                    pap = v1[0];
+                    if constexpr (kOneWarpSums<A>) {
+                        onewarp_send<A, 1>(v1, slots, wscr, 0, tx, C, rank, PTRI ? halo_in : 0u);
+                        const ReduceOut *o = onewarp_finish<A, 1>(
+                            v1, slots, 0, tx, C, [&](int, A s, ReduceOut *out) { onewarp_alpha<T>(s, eta, out, tid & 31); });
+                        alpha = *reinterpret_cast<const T *>(&o->ratio);
+                        code1 = o->code[0];
+                        pap = v1[0];
+                    } else {
+                        solver_allreduce<A, 1>(v1, slots, wscr, 0, tx, cluster, C, rank, PTRI ? halo_in : 0u);
+                        pap = v1[0];
+                        alpha = (pap == A(0)) ? T(0) : acc_ratio<T>(eta, pap);
+                    }
                 }
-                const T alpha = (pap == A(0)) ? T(0) : acc_ratio<T>(eta, pap);
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) {
                     lam[q] = fma_rn(alpha, p[q], lam[q]);
@@ -1378,6 +1545,8 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                 matP_rows(z);
                 if (first_knot) push_halo_tx<T, RPT>(zh + NP + i, rank - 1, z, tx, 1);
                 if (last_knot) push_halo_tx<T, RPT>(zh + i, rank + 1, z, tx, 1);
+                T beta_h = T(0);
+                uint32_t code2 = 0;
                 {
                     A v2[2] = {A(0), A(0)};
 #pragma unroll
@@ -1385,14 +1554,31 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                         acc_madd(v2[0], r[q], z[q]);
                         if (relres) acc_madd(v2[1], r[q], r[q]);
                     }
-                    solver_allreduce<A, 2>(v2, slots, wscr, 1, tx, cluster, C, rank, halo_in);
+                    if constexpr (kOneWarpSums<A>) {
+                        onewarp_send<A, 2>(v2, slots, wscr, 1, tx, C, rank, halo_in);
+                        const ReduceOut *o = onewarp_finish<A, 2>(
+                            v2, slots, 1, tx, C,
+                            [&](int q, A s, ReduceOut *out) { onewarp_beta<T>(q, s, eta, tol, thr, out, tid & 31); });
+                        beta_h = *reinterpret_cast<const T *>(&o->ratio);
+                        code1 |= o->code[0] & kNotFinite;
+                        code2 = o->code[relres ? 1 : 0];
+                    } else {
+                        solver_allreduce<A, 2>(v2, slots, wscr, 1, tx, cluster, C, rank, halo_in);
+                    }
                     eta_new = v2[0];
                     rr = v2[1];
                 }
                 ++iter;
-                if (!acc_finite(eta_new) || !acc_finite(pap)) { status = ST_BREAKDOWN; break; }
-                if (relres ? (rr <= thr) : (acc_abs(eta_new) < tol)) { status = ST_CONVERGED; break; }
-                const T beta = acc_ratio<T>(eta_new, eta);
+                T beta;
+                if constexpr (kOneWarpSums<A>) {
+                    if (code1 & kNotFinite) { status = ST_BREAKDOWN; break; }
+                    if (code2 & kExitTest) { status = ST_CONVERGED; break; }
+                    beta = beta_h;
+                } else {
+                    if (!acc_finite(eta_new) || !acc_finite(pap)) { status = ST_BREAKDOWN; break; }
+                    if (relres ? (rr <= thr) : (acc_abs(eta_new) < tol)) { status = ST_CONVERGED; break; }
+                    beta = acc_ratio<T>(eta_new, eta);
+                }
                 eta = eta_new;
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) {

@@ -274,6 +274,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) pcg_stream_kernel(const Lau
         const uint32_t max_iter = d.max_iter;
         for (; iter < max_iter;) {
             A pap;
+            T alpha, beta_h = T(0);
+            uint32_t code1 = 0, code2 = 0;
             {
                 A v1[1] = {A(0)};
                 for (uint32_t g = 0; g < G; ++g) {
@@ -291,10 +293,19 @@ __global__ void __launch_bounds__(kStreamThreads, 1) pcg_stream_kernel(const Lau
                         if (s.last) push_halo_tx<T, RPT>(uh + s.i, rank + 1, y, tx, 0);
                     }
                 }
-                solver_allreduce<A, 1>(v1, slots, wscr, 0, tx, cluster, C, rank, PTRI ? halo_in : 0u);
-                pap = v1[0];
+                if constexpr (kOneWarpSums<A>) {
+                    onewarp_send<A, 1>(v1, slots, wscr, 0, tx, C, rank, PTRI ? halo_in : 0u);
+                    const ReduceOut *o = onewarp_finish<A, 1>(
+                        v1, slots, 0, tx, C, [&](int, A s, ReduceOut *out) { onewarp_alpha<T>(s, eta, out, tid & 31); });
+                    alpha = *reinterpret_cast<const T *>(&o->ratio);
+                    code1 = o->code[0];
+                    pap = v1[0];
+                } else {
+                    solver_allreduce<A, 1>(v1, slots, wscr, 0, tx, cluster, C, rank, PTRI ? halo_in : 0u);
+                    pap = v1[0];
+                    alpha = (pap == A(0)) ? T(0) : acc_ratio<T>(eta, pap);
+                }
             }
-            const T alpha = (pap == A(0)) ? T(0) : acc_ratio<T>(eta, pap);
             for (uint32_t g = 0; g < G; ++g) {
                 const Slot s = slot(g);
                 if (!s.act) continue;
@@ -333,14 +344,31 @@ __global__ void __launch_bounds__(kStreamThreads, 1) pcg_stream_kernel(const Lau
                     if (s.first) push_halo_tx<T, RPT>(zh + NP + s.i, rank - 1, z, tx, 1);
                     if (s.last) push_halo_tx<T, RPT>(zh + s.i, rank + 1, z, tx, 1);
                 }
-                solver_allreduce<A, 2>(v2, slots, wscr, 1, tx, cluster, C, rank, halo_in);
+                if constexpr (kOneWarpSums<A>) {
+                    onewarp_send<A, 2>(v2, slots, wscr, 1, tx, C, rank, halo_in);
+                    const ReduceOut *o = onewarp_finish<A, 2>(
+                        v2, slots, 1, tx, C,
+                        [&](int q, A s, ReduceOut *out) { onewarp_beta<T>(q, s, eta, tol, thr, out, tid & 31); });
+                    beta_h = *reinterpret_cast<const T *>(&o->ratio);
+                    code1 |= o->code[0] & kNotFinite;
+                    code2 = o->code[relres ? 1 : 0];
+                } else {
+                    solver_allreduce<A, 2>(v2, slots, wscr, 1, tx, cluster, C, rank, halo_in);
+                }
                 eta_new = v2[0];
                 rr = v2[1];
             }
             ++iter;
-            if (!acc_finite(eta_new) || !acc_finite(pap)) { status = ST_BREAKDOWN; break; }
-            if (relres ? (rr <= thr) : (acc_abs(eta_new) < tol)) { status = ST_CONVERGED; break; }
-            const T beta = acc_ratio<T>(eta_new, eta);
+            T beta;
+            if constexpr (kOneWarpSums<A>) {
+                if (code1 & kNotFinite) { status = ST_BREAKDOWN; break; }
+                if (code2 & kExitTest) { status = ST_CONVERGED; break; }
+                beta = beta_h;
+            } else {
+                if (!acc_finite(eta_new) || !acc_finite(pap)) { status = ST_BREAKDOWN; break; }
+                if (relres ? (rr <= thr) : (acc_abs(eta_new) < tol)) { status = ST_CONVERGED; break; }
+                beta = acc_ratio<T>(eta_new, eta);
+            }
             eta = eta_new;
             for (uint32_t g = 0; g < G; ++g) {
                 const Slot s = slot(g);
