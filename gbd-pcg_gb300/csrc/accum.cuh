@@ -29,6 +29,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stdint.h>
 
 #include <type_traits>
 
@@ -93,6 +94,31 @@ __device__ __forceinline__ void acc_madd(A &v, T a, T b) {
     }
 }
 
+// float(a / b) of two doubles without the FP64 pipe (a double division is about
+// ten dependent FP64 instructions): the operands' mantissas as float pairs, one
+// float division, one correction with the remainder (as for f2acc below), and
+// the exponents put back.  Within 2^-45 of the quotient before its rounding to
+// float; zeros, subnormals, non-finite operands and quotients near or past the
+// range of float go through the double division.
+__device__ __forceinline__ float ratio_f32(double a, double b) {
+    const uint32_t ah = (uint32_t)__double2hiint(a), bh = (uint32_t)__double2hiint(b);
+    const uint32_t al = (uint32_t)__double2loint(a), bl = (uint32_t)__double2loint(b);
+    const int ea = (int)((ah >> 20) & 0x7ffu), eb = (int)((bh >> 20) & 0x7ffu), k = ea - eb;
+    if (ea == 0 || eb == 0 || ea == 0x7ff || eb == 0x7ff || k > 120 || k < -120) return (float)(a / b);
+    // mantissa in [1, 2): the leading 23 bits as a float, the other 29 scaled by 2^-52
+    const float a0 = __uint_as_float(0x3f800000u | ((ah & 0xfffffu) << 3) | (al >> 29));
+    const float b0 = __uint_as_float(0x3f800000u | ((bh & 0xfffffu) << 3) | (bl >> 29));
+    const float a1 = __fmul_rn((float)(al & 0x1fffffffu), 2.220446049250313e-16f);
+    const float b1 = __fmul_rn((float)(bl & 0x1fffffffu), 2.220446049250313e-16f);
+    const float q = __fdiv_rn(a0, b0);
+    float r = __fmaf_rn(-q, b0, a0);  // exact
+    r = __fadd_rn(r, a1);
+    r = __fmaf_rn(-q, b1, r);
+    const float v = __fadd_rn(q, __fdiv_rn(r, b0));
+    // 2^k with the quotient's sign
+    return __fmul_rn(v, __uint_as_float(((ah ^ bh) & 0x80000000u) | ((uint32_t)(k + 127) << 23)));
+}
+
 // T(a / b)
 template <typename T, typename A>
 __device__ __forceinline__ T acc_ratio(const A &a, const A &b) {
@@ -102,6 +128,8 @@ __device__ __forceinline__ T acc_ratio(const A &a, const A &b) {
         r = __fadd_rn(r, a.lo);
         r = __fmaf_rn(-q, b.lo, r);
         return T(__fadd_rn(q, __fdiv_rn(r, b.hi)));
+    } else if constexpr (std::is_same<A, double>::value && std::is_same<T, float>::value) {
+        return ratio_f32(a, b);
     } else {
         return T(a / b);
     }

@@ -286,6 +286,24 @@ bool plain_fits(Registry *reg, bool f64, uint32_t n, uint32_t N) {
     return (int64_t)per_sm * reg->sm_count >= (int64_t)N;
 }
 
+// CTAs of a shape that one SM holds at once: its registers (64K in four
+// sub-partitions, whole warps of a multiple of 8 registers a thread) and its
+// shared memory.
+uint32_t ctas_per_sm(const Shape &s) {
+    const uint32_t regs = (uint32_t)(s.vi->regs + 7) / 8 * 8, warps = (s.threads / 32 + 3) / 4 * 4;
+    const uint32_t by_regs = 65536u / (regs * 32u * warps);
+    const size_t smem = s.vi->v.smem_bytes(s.K, s.C, s.threads / 32) + 1024;
+    return std::min<uint32_t>(by_regs, (uint32_t)(228u * 1024u / smem));
+}
+
+// Tensor-memory rows against the storage the preference order finds, for
+// batches: a tensor-memory CTA has its SM to itself, so it pays where the
+// other storage's CTA would have it to itself too (its registers fit the SM
+// once), and not where several of those would share the SM.  Refinement,
+// measured: 256 x n=24 N=256 with C 8 against 16, 91 against 181 ms; 64 x n=24
+// N=64 5.6 / 8.7; 200 x n=14 N=100 16.7 / 19.3; 32 x n=14 N=32 3.74 / 3.95;
+// on the other side 256 x n=8 N=32 (three CTAs of split rows an SM) 4.7 / 3.6.
+//
 // c_pref > 1 (lone systems, cluster size not pinned): clusters from c_pref up
 // are tried first, then the smallest that fits.  `lone`: a single system
 // solved by itself.  For such a system with a cbtd Phi^-1 that no on-chip
@@ -330,6 +348,36 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
     // 1.4-1.6 us with S in registers and Phi^-1 in shared memory).
     if (lone && cfg.storage == GBDPCG_STORAGE_AUTO && !f64 && !refine && !ptri)
         prefs.insert(prefs.begin(), Pref{4, 2});
+    // the first cluster size from `from` up at which storage pf holds the system
+    auto fit = [&](const Pref &pf, uint32_t from, Shape *o) -> bool {
+        if (pf.rpt > 1 && (n % pf.rpt) != 0) return false;
+        VariantInfo *vi = find_variant(reg, f64 && !refine, acc, np, ptri, pf.st, pf.rpt, alg, fa);
+        if (!vi) return false;
+        uint32_t cap = cfg.max_threads ? cfg.max_threads : (uint32_t)vi->max_threads;
+        cap = std::min<uint32_t>(cap, (uint32_t)vi->max_threads);
+        const uint32_t c_lo = cfg.cluster_size ? cfg.cluster_size : from;
+        const uint32_t c_hi = cfg.cluster_size ? cfg.cluster_size : 16;
+        for (uint32_t C = c_lo; C <= c_hi; ++C) {
+            if (C > 8 && (C & (C - 1))) continue;  // large clusters: powers of two only
+            const uint32_t K = (N + C - 1) / C;
+            const uint32_t thr = (K * n + pf.rpt - 1) / pf.rpt;
+            if (thr > cap && !streamed(pf.st)) continue;
+            // CTA sizes are rounded to 64 threads so that systems of similar
+            // size share a launch (streamed rows: up to the cap, in row groups)
+            uint32_t threads = std::min<uint32_t>(cap, std::max<uint32_t>(64, (thr + 63) / 64 * 64));
+            if (threads < thr && !streamed(pf.st)) threads = (thr + 31) / 32 * 32;
+            // shared memory at the largest CTA the class may get (streamed rows:
+            // at this CTA, whose vectors are what bound the system)
+            const uint32_t chk_warps = streamed(pf.st) ? threads / 32 : 32;
+            if (vi->v.smem_bytes(K, C, chk_warps) > (size_t)reg->max_smem_optin) continue;
+            o->vi = vi;
+            o->C = C;
+            o->K = K;
+            o->threads = threads;
+            return true;
+        }
+        return false;
+    };
     for (uint32_t from : {first_lo, 1u}) {
         for (const Pref &pf : prefs) {
             if (pf.rpt > 1 && (n % pf.rpt) != 0) continue;
@@ -339,32 +387,13 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
                 *out = s;
                 return GBDPCG_SUCCESS;
             }
-            VariantInfo *vi = find_variant(reg, f64 && !refine, acc, np, ptri, pf.st, pf.rpt, alg, fa);
-            if (!vi) continue;
-            uint32_t cap = cfg.max_threads ? cfg.max_threads : (uint32_t)vi->max_threads;
-            cap = std::min<uint32_t>(cap, (uint32_t)vi->max_threads);
-            const uint32_t c_lo = cfg.cluster_size ? cfg.cluster_size : from;
-            const uint32_t c_hi = cfg.cluster_size ? cfg.cluster_size : 16;
-            for (uint32_t C = c_lo; C <= c_hi; ++C) {
-                if (C > 8 && (C & (C - 1))) continue;  // large clusters: powers of two only
-                const uint32_t K = (N + C - 1) / C;
-                const uint32_t thr = (K * n + pf.rpt - 1) / pf.rpt;
-                if (thr > cap && !streamed(pf.st)) continue;
-                // CTA sizes are rounded to 64 threads so that systems of similar
-                // size share a launch (streamed rows: up to the cap, in row groups)
-                uint32_t threads = std::min<uint32_t>(cap, std::max<uint32_t>(64, (thr + 63) / 64 * 64));
-                if (threads < thr && !streamed(pf.st)) threads = (thr + 31) / 32 * 32;
-                // shared memory at the largest CTA the class may get (streamed rows:
-                // at this CTA, whose vectors are what bound the system)
-                const uint32_t chk_warps = streamed(pf.st) ? threads / 32 : 32;
-                if (vi->v.smem_bytes(K, C, chk_warps) > (size_t)reg->max_smem_optin) continue;
-                s.vi = vi;
-                s.C = C;
-                s.K = K;
-                s.threads = threads;
-                *out = s;
-                return GBDPCG_SUCCESS;
+            if (!fit(pf, from, &s)) continue;
+            if (refine && cfg.storage == GBDPCG_STORAGE_AUTO && ctas_per_sm(s) < 2) {
+                Shape t;
+                if (fit(Pref{4, 2}, from, &t) && t.C <= s.C) s = t;
             }
+            *out = s;
+            return GBDPCG_SUCCESS;
         }
         if (from == 1) break;  // the second pass would repeat the first
     }

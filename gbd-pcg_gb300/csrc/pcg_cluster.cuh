@@ -879,15 +879,19 @@ __device__ __forceinline__ void onewarp_send(A (&v)[NQ], A *slots, A *wscr, int 
     for (int q = 0; q < NQ; ++q) {
         if (warp != (uint32_t)q % nwarps) continue;
         const A *x = wscr + (uint32_t)q * nwarps * 32 + lane;
-        A t[1] = {x[0]}, t1 = A(0);
+        A t[1] = {x[0]}, c[3] = {A(0), A(0), A(0)};  // four chains
         uint32_t w = 1;
-#pragma unroll 4
-        for (; w + 1 < nwarps; w += 2) {
-            t[0] += x[w * 32];
-            t1 += x[w * 32 + 32];
+        if (nwarps >= 4) {
+#pragma unroll
+            for (int u = 0; u < 3; ++u) c[u] = x[(w + u) * 32];
+            for (w = 4; w + 4 <= nwarps; w += 4) {
+                t[0] += x[w * 32];
+#pragma unroll
+                for (int u = 0; u < 3; ++u) c[u] += x[(w + 1 + u) * 32];
+            }
         }
-        if (w < nwarps) t[0] += x[w * 32];
-        if (nwarps > 2) t[0] += t1;
+        for (; w < nwarps; ++w) t[0] += x[w * 32];
+        if (nwarps >= 4) t[0] = (t[0] + c[0]) + (c[1] + c[2]);
         warp_sum_n<A, 1>(t);
         v[q] = t[0];
         if (C > 1 && lane < C) {

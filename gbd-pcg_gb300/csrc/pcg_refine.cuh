@@ -4,7 +4,8 @@
 //
 // Per system (one cluster, knots split over its CTAs as in pcg_cluster.cuh):
 //   * the rows of S are converted once from the FP64 input to FP32 and held on
-//     chip (registers or shared memory), Phi^-1 is FP32 block-diagonal;
+//     chip (registers, shared memory or tensor memory), Phi^-1 is FP32
+//     block-diagonal;
 //   * lambda and gamma stay FP64 in registers;
 //   * outer step: r64 = gamma - S64 lambda64, with S64 read from global memory
 //     (FP64 FMAs, lambda halo through DSMEM), ||r64|| reduced in FP64; stop when
@@ -13,6 +14,14 @@
 //     ||r_inner|| <= inner_tol ||r64||, its dot products accumulated in AI:
 //     double, or f2acc (float-float, on the FP32 pipe; see accum.cuh);
 //   * lambda64 += d.
+// What bounds it: the inner iteration's chain of products and reductions on the
+// SMs that hold one system, and beside it the FP64 pipe (2 lanes a clock per
+// SM), which the inner dot products share with every reduction.  So a system
+// takes as few SMs as hold its rows (tensor memory: 768 rows of n = 24 an SM,
+// against 512 in registers and shared memory), the reductions are the
+// transaction-counted ones of the cluster kernel with one summing warp per
+// value, and the factors of a product are widened to FP64 by integer
+// operations (conversions run at the FP64 pipe's rate).
 // Result: iters = inner PCG passes summed over the outer steps, outer = outer
 // steps, rr = the final ||r64||^2.
 #pragma once
@@ -31,13 +40,34 @@ struct SmemPlanRF {
     }
 };
 
+// x as a double, exactly.  F2F.F64.F32 issues at the FP64 pipe's rate (2 lanes a
+// clock per SM); for normal numbers the widening is a shift of the mantissa and
+// a new exponent bias (895 + 1 = 1023 - 127), on the integer pipe.
+__device__ __forceinline__ double widen(float x) {
+    const uint32_t u = __float_as_uint(x), e = u & 0x7f800000u;
+    if (e == 0u || e == 0x7f800000u) return (u << 1) == 0u ? __hiloint2double((int)u, 0) : (double)x;
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+
+// v += a b of the inner dot products
+template <typename AI>
+__device__ __forceinline__ void inner_madd(AI &v, float a, float b) {
+    if constexpr (std::is_same<AI, double>::value) v = fma(widen(a), widen(b), v);
+    else acc_madd(v, a, b);
+}
+
 template <int NP, int ST, int RPT, typename AI>
 __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>::max_threads), 1)
     pcg_refine_kernel(const LaunchParams lp) {
     using T = float;
     static_assert(sizeof(AI) == sizeof(double), "inner and outer reductions share the slot arrays");
     using Plan = SmemPlan<T, double, NP, false, ST>;
-    constexpr bool S_REG = ST <= ST_REG_S, P_REG = ST == ST_REG;
+    constexpr bool S_REG = ST <= ST_REG_S, P_REG = ST == ST_REG, S_TM = ST == ST_TMEM;
+    static_assert(!S_TM || RPT == 2, "tensor-memory storage: two rows per thread");
+    constexpr int NPT = tmem_cols<NP>();
+    static_assert(!S_TM || (RegBudget<float, double, NP, false, ST, RPT>::max_threads + 127) / 128 * RPT * 3 * NPT <=
+                               (int)kTmemColumns,
+                  "the warps of a CTA fit the tensor memory's columns");
     const cg::cluster_group cluster = cg::this_cluster();
     const uint32_t C = cluster.num_blocks();
     const uint32_t rank = cluster.block_rank();
@@ -52,7 +82,8 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
     double *slots64 = reinterpret_cast<double *>(sp); sp += Plan::slots(C);  // FP64 reductions
     double *wscr64 = reinterpret_cast<double *>(sp); sp += Plan::wscr(nthr >> 5);
     AI *slots = reinterpret_cast<AI *>(slots64);  // the same bytes for the inner reductions
-    AI *wscr = reinterpret_cast<AI *>(wscr64);
+    // float-float partials behind the one row of partials the FP64 reductions use
+    AI *wscr = reinterpret_cast<AI *>(wscr64) + (kOneWarpSums<AI> ? 0u : nthr);
     uint32_t *s_item = reinterpret_cast<uint32_t *>(sp); sp += kItemBytes;
     T *ms = reinterpret_cast<T *>(sp); sp += Plan::mat_s(lp.kmax);
     T *mp = reinterpret_cast<T *>(sp); sp += Plan::mat_p(lp.kmax);
@@ -62,7 +93,28 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
     const uint32_t zero_d = (uint32_t)(SmemPlanRF<NP, ST>::dwin(lp.kmax) / sizeof(double));
 
     for (uint32_t e = tid; e < (uint32_t)(Plan::slots(C) / sizeof(double)); e += nthr) slots64[e] = 0.0;
-    for (uint32_t e = tid; e < (uint32_t)(kMaxValues * 32); e += nthr) wscr64[e] = 0.0;  // local slots
+    for (uint32_t e = tid; e < (uint32_t)kMaxValues * nthr; e += nthr) wscr64[e] = 0.0;  // local slots
+    TxReduce tx{reinterpret_cast<uint64_t *>(s_item + 8), 0u, s_item + 12};
+    if (C > 1) {
+        if (tid == 0) {
+            mbar_init(tx.bar, 1);
+            mbar_init(tx.bar + 1, 1);
+            *tx.timed_out = 0u;
+            mbar_init_fence();
+        }
+        cluster.sync();
+    } else {
+        __syncthreads();
+    }
+    uint32_t tbase = 0, trow = 0;  // tensor memory, as in pcg_cluster_kernel
+    if constexpr (S_TM) {
+        if ((tid >> 5) == 0) tmem_alloc(s_item + 1, kTmemColumns);
+        tmem_fence_before_sync();
+        __syncthreads();
+        tmem_fence_after_sync();
+        tbase = *reinterpret_cast<volatile uint32_t *>(s_item + 1);
+        trow = tbase + ((((tid >> 5) & 3u) * 32u) << 16) + (tid >> 7) * (uint32_t)(RPT * 3 * NPT);
+    }
     const uint32_t cluster_id = blockIdx.x / C, nclusters = gridDim.x / C;
     Stamper stamp(lp, rank);
     for (uint32_t pass = 0;; ++pass) {
@@ -110,6 +162,8 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
         const bool has_left = nk > 0 && kb > 0, has_right = nk > 0 && ke < N;
         const bool first_knot = act && lk == 0 && kb > 0, last_knot = act && lk + 1 == nk && ke < N;
         const int sb0 = (k == 0) ? 1 : 0, sb1 = (k + 1 == N) ? 2 : 3;
+        // halo bytes the neighbours send to this CTA before a reduction (n values each)
+        const uint32_t halo_in = ((has_left ? n : 0u) + (has_right ? n : 0u)) * (uint32_t)sizeof(T);
         if (tid == 0 && nk > 0) {  // this CTA's rows into L2 before they are staged
             prefetch_l2_range(S64 + (size_t)kb * blkS, (size_t)nk * blkS * sizeof(double));
             prefetch_l2_range(P + (size_t)kb * blkP, (size_t)nk * blkP * sizeof(T));
@@ -119,7 +173,7 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
         for (uint32_t e = tid; e < zero_d; e += nthr) vd[e] = 0.0;
 
         // ---- FP32 copies of the rows of S (converted once), FP32 Phi^-1
-        T Sr[S_REG ? RPT : 1][S_REG ? 3 * NP : 1];
+        T Sr[S_REG || S_TM ? RPT : 1][S_REG ? 3 * NP : (S_TM ? NP : 1)];
         T Pr[P_REG ? RPT : 1][P_REG ? NP : 1];
         if constexpr (S_REG) {
             const double *Sk = S64 + (size_t)k * blkS;
@@ -134,11 +188,44 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
                                                 ? __double2float_rn(__ldg(Sk + (b * n + j) * n + i + q))
                                                 : T(0);
             }
+        } else if constexpr (S_TM) {
+            // the diagonal block in registers; the off-diagonal blocks and Phi^-1
+            // to tensor memory, 8 columns of a row at a time
+            const double *Sk = S64 + (size_t)k * blkS;
+            const T *Pk = P + (size_t)k * blkP;
+#pragma unroll
+            for (int j = 0; j < NP; ++j)
+#pragma unroll
+                for (int q = 0; q < RPT; ++q)
+                    Sr[q][j] = (act && (uint32_t)j < n) ? __double2float_rn(__ldg(Sk + (n + j) * n + i + q)) : T(0);
+            __syncwarp();  // tcgen05 stores are warp-wide
+#pragma unroll
+            for (int bi = 0; bi < 3; ++bi) {
+                const bool present = act && (bi != 0 || k > 0) && (bi != 1 || k + 1 < N);
+#pragma unroll
+                for (int q = 0; q < RPT; ++q)
+#pragma unroll
+                    for (int cc = 0; cc < NPT / 8; ++cc) {
+                        float v[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            const uint32_t j = 8 * cc + u;
+                            v[u] = 0.f;
+                            if (present && j < n)
+                                v[u] = bi == 2 ? __ldg(Pk + (size_t)j * n + i + q)
+                                               : __double2float_rn(__ldg(Sk + ((size_t)(2 * bi) * n + j) * n + i + q));
+                        }
+                        tmem_st8(trow + (uint32_t)((q * 3 + bi) * NPT + 8 * cc), v);
+                    }
+            }
+            tmem_wait_st();
         } else {
             const double *Sg = S64 + (size_t)kb * blkS;
             stage_rows(ms, R, Sg, nk, n, blkS, tid, nthr);
         }
-        if constexpr (P_REG) {
+        if constexpr (S_TM) {
+            // Phi^-1 went to tensor memory with the off-diagonal S blocks
+        } else if constexpr (P_REG) {
             const T *Pk = P + (size_t)k * blkP;
 #pragma unroll
             for (int j = 0; j < NP; ++j)
@@ -149,13 +236,29 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
             const T *Pg = P + (size_t)kb * blkP;
             stage_rows(mp, R, Pg, nk, n, blkP, tid, nthr);
         }
+        // S x and Phi^-1 x over this thread's rows (zero for a thread without rows);
+        // with tensor memory every thread of a warp takes part in the loads
         auto matS = [&](const T *x, T(&y)[RPT]) {
-            if constexpr (S_REG) reg_matvec<T, NP, 3, RPT>(Sr, x, y);
-            else smem_matvec<T, NP, 3, RPT>(ms, R, lk * n + i, sb0, sb1, x, n, y);
+            if constexpr (S_TM) tmem_matvec<NP>(Sr, trow, x + (act ? lk : 0u) * NP, y);
+            else if (act) {
+                if constexpr (S_REG) reg_matvec<T, NP, 3, RPT>(Sr, x + lk * NP, y);
+                else smem_matvec<T, NP, 3, RPT>(ms, R, lk * n + i, sb0, sb1, x + lk * NP, n, y);
+            }
+            if (!act) {
+#pragma unroll
+                for (int q = 0; q < RPT; ++q) y[q] = T(0);
+            }
         };
         auto matP = [&](const T *x, T(&y)[RPT]) {
-            if constexpr (P_REG) reg_matvec<T, NP, 1, RPT>(Pr, x + NP, y);
-            else smem_matvec<T, NP, 1, RPT>(mp, R, lk * n + i, 0, 1, x + NP, n, y);
+            if constexpr (S_TM) tmem_pmatvec<NP>(trow, x + (act ? lk : 0u) * NP, y);
+            else if (act) {
+                if constexpr (P_REG) reg_matvec<T, NP, 1, RPT>(Pr, x + (lk + 1) * NP, y);
+                else smem_matvec<T, NP, 1, RPT>(mp, R, lk * n + i, 0, 1, x + (lk + 1) * NP, n, y);
+            }
+            if (!act) {
+#pragma unroll
+                for (int q = 0; q < RPT; ++q) y[q] = T(0);
+            }
         };
         T *my_p = vp + (lk + 1) * NP + i;
         T *my_r = vr + (lk + 1) * NP + i;
@@ -176,7 +279,7 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
             double v1[1] = {0.0};
 #pragma unroll
             for (int q = 0; q < RPT; ++q) v1[0] = fma(gam[q], gam[q], v1[0]);
-            cluster_allreduce<double, 1>(v1, slots64, wscr64, buf, cluster, C, rank);
+            solver_allreduce<double, 1>(v1, slots64, wscr64, buf, tx, cluster, C, rank, 0u);
             buf ^= 1;
             gg = v1[0];
         }
@@ -223,7 +326,7 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
                 double v1[1] = {0.0};
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) v1[0] = fma(r64[q], r64[q], v1[0]);
-                cluster_allreduce<double, 1>(v1, slots64, wscr64, buf, cluster, C, rank);
+                solver_allreduce<double, 1>(v1, slots64, wscr64, buf, tx, cluster, C, rank, 0u);
                 buf ^= 1;
                 rr64 = v1[0];
             }
@@ -240,35 +343,23 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
                 if (act) my_r[q] = r[q];
             }
             __syncthreads();
-            if (act) matP(vr + lk * NP, z);
-            else {
-#pragma unroll
-                for (int q = 0; q < RPT; ++q) z[q] = T(0);
-            }
+            matP(vr, z);
 #pragma unroll
             for (int q = 0; q < RPT; ++q) {
                 p[q] = z[q];
                 if (act) my_p[q] = p[q];
             }
-            if (first_knot) {
-                T *dst = cluster.map_shared_rank(vp, rank - 1) + (K + 1) * NP + i;
-#pragma unroll
-                for (int q = 0; q < RPT; ++q) dst[q] = z[q];
-            }
-            if (last_knot) {
-                T *dst = cluster.map_shared_rank(vp, rank + 1) + i;
-#pragma unroll
-                for (int q = 0; q < RPT; ++q) dst[q] = z[q];
-            }
+            if (first_knot) push_halo_tx<T, RPT>(vp + (K + 1) * NP + i, rank - 1, z, tx, buf);
+            if (last_knot) push_halo_tx<T, RPT>(vp + i, rank + 1, z, tx, buf);
             AI eta, rr_in0;
             {
                 AI v2[2] = {AI(0), AI(0)};
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) {
-                    acc_madd(v2[0], r[q], z[q]);
-                    acc_madd(v2[1], r[q], r[q]);
+                    inner_madd(v2[0], r[q], z[q]);
+                    inner_madd(v2[1], r[q], r[q]);
                 }
-                cluster_allreduce<AI, 2>(v2, slots, wscr, buf, cluster, C, rank);
+                solver_allreduce<AI, 2>(v2, slots, wscr, buf, tx, cluster, C, rank, halo_in);
                 buf ^= 1;
                 eta = v2[0];
                 rr_in0 = v2[1];
@@ -278,21 +369,28 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
             uint32_t it = 0;
             bool broke = false;
             for (; it < budget;) {
-                if (act) matS(vp + lk * NP, y);
-                else {
-#pragma unroll
-                    for (int q = 0; q < RPT; ++q) y[q] = T(0);
-                }
+                matS(vp, y);
                 AI pap;
+                T alpha, beta;
+                uint32_t code1 = 0, code2 = 0;
                 {
                     AI v1[1] = {AI(0)};
 #pragma unroll
-                    for (int q = 0; q < RPT; ++q) acc_madd(v1[0], p[q], y[q]);
-                    cluster_allreduce<AI, 1>(v1, slots, wscr, buf, cluster, C, rank);
-                    buf ^= 1;
+                    for (int q = 0; q < RPT; ++q) inner_madd(v1[0], p[q], y[q]);
+                    if constexpr (kOneWarpSums<AI>) {
+                        onewarp_send<AI, 1>(v1, slots, wscr, buf, tx, C, rank, 0u);
+                        const ReduceOut *o = onewarp_finish<AI, 1>(
+                            v1, slots, buf, tx, C,
+                            [&](int, AI s, ReduceOut *out) { onewarp_alpha<T>(s, eta, out, tid & 31); });
+                        alpha = *reinterpret_cast<const T *>(&o->ratio);
+                        code1 = o->code[0];
+                    } else {
+                        solver_allreduce<AI, 1>(v1, slots, wscr, buf, tx, cluster, C, rank, 0u);
+                        alpha = (v1[0] == AI(0)) ? T(0) : acc_ratio<T>(eta, v1[0]);
+                    }
                     pap = v1[0];
+                    buf ^= 1;
                 }
-                const T alpha = (pap == AI(0)) ? T(0) : acc_ratio<T>(eta, pap);
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) {
                     x[q] = fma_rn(alpha, p[q], x[q]);
@@ -300,39 +398,42 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
                     if (act) my_r[q] = r[q];
                 }
                 __syncthreads();
-                if (act) matP(vr + lk * NP, z);
-                else {
-#pragma unroll
-                    for (int q = 0; q < RPT; ++q) z[q] = T(0);
-                }
-                if (first_knot) {
-                    T *dst = cluster.map_shared_rank(zh, rank - 1) + NP + i;
-#pragma unroll
-                    for (int q = 0; q < RPT; ++q) dst[q] = z[q];
-                }
-                if (last_knot) {
-                    T *dst = cluster.map_shared_rank(zh, rank + 1) + i;
-#pragma unroll
-                    for (int q = 0; q < RPT; ++q) dst[q] = z[q];
-                }
+                matP(vr, z);
+                if (first_knot) push_halo_tx<T, RPT>(zh + NP + i, rank - 1, z, tx, buf);
+                if (last_knot) push_halo_tx<T, RPT>(zh + i, rank + 1, z, tx, buf);
                 AI eta_new, rr;
                 {
                     AI v2[2] = {AI(0), AI(0)};
 #pragma unroll
                     for (int q = 0; q < RPT; ++q) {
-                        acc_madd(v2[0], r[q], z[q]);
-                        acc_madd(v2[1], r[q], r[q]);
+                        inner_madd(v2[0], r[q], z[q]);
+                        inner_madd(v2[1], r[q], r[q]);
                     }
-                    cluster_allreduce<AI, 2>(v2, slots, wscr, buf, cluster, C, rank);
+                    if constexpr (kOneWarpSums<AI>) {
+                        onewarp_send<AI, 2>(v2, slots, wscr, buf, tx, C, rank, halo_in);
+                        const ReduceOut *o = onewarp_finish<AI, 2>(
+                            v2, slots, buf, tx, C,
+                            [&](int q, AI s, ReduceOut *out) { onewarp_beta<T>(q, s, eta, AI(0), thr_in, out, tid & 31); });
+                        beta = *reinterpret_cast<const T *>(&o->ratio);
+                        code1 |= o->code[0] & kNotFinite;
+                        code2 = o->code[1];
+                    } else {
+                        solver_allreduce<AI, 2>(v2, slots, wscr, buf, tx, cluster, C, rank, halo_in);
+                    }
                     buf ^= 1;
                     eta_new = v2[0];
                     rr = v2[1];
                 }
                 ++it;
                 eta_last = eta_new;
-                if (!acc_finite(eta_new) || !acc_finite(pap)) { broke = true; break; }
-                if (rr <= thr_in) break;
-                const T beta = acc_ratio<T>(eta_new, eta);
+                if constexpr (kOneWarpSums<AI>) {
+                    if (code1 & kNotFinite) { broke = true; break; }
+                    if (code2 & kExitTest) break;
+                } else {
+                    if (!acc_finite(eta_new) || !acc_finite(pap)) { broke = true; break; }
+                    if (rr <= thr_in) break;
+                    beta = acc_ratio<T>(eta_new, eta);
+                }
                 eta = eta_new;
 #pragma unroll
                 for (int q = 0; q < RPT; ++q) {
@@ -362,6 +463,9 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
             for (int q = 0; q < RPT; ++q) lam_out[(size_t)k * n + i + q] = lam[q];
         }
         if (rank == 0 && tid == 0) {
+            if (C > 1)  // a reduction wait of some CTA of the cluster gave up
+                for (uint32_t c = 0; c < C; ++c)
+                    if (*cluster.map_shared_rank(tx.timed_out, c)) status = ST_TIMEOUT;
             SysResult res;
             res.iters = iters;
             res.status = status;
@@ -373,6 +477,13 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
             lp.results[d.result] = res;
         }
         stamp.done(lp, item, iters);
+    }
+    if (C > 1) cluster.sync();  // every transaction-counted store into this CTA has landed
+    if constexpr (S_TM) {
+        tmem_fence_before_sync();
+        __syncthreads();
+        tmem_fence_after_sync();
+        if ((tid >> 5) == 0) tmem_dealloc(tbase, kTmemColumns);
     }
 }
 

@@ -46,7 +46,9 @@
     out[c++] = GBDPCG_VARIANT_RF(NP, ST_REG, 1);                                              \
     out[c++] = GBDPCG_VARIANT_RF(NP, ST_REG_S, 1);                                            \
     out[c++] = GBDPCG_VARIANT_RF(NP, ST_SMEM, 1);
-#define GBDPCG_VARIANTS_RF_RPT2(NP) out[c++] = GBDPCG_VARIANT_RF(NP, ST_REG_S, 2);
+#define GBDPCG_VARIANTS_RF_RPT2(NP)                                                           \
+    out[c++] = GBDPCG_VARIANT_RF(NP, ST_REG_S, 2);                                            \
+    out[c++] = GBDPCG_VARIANT_RF(NP, ST_TMEM, 2);
 
 // FP32: rows in registers (RPT 1; RPT 2 for even bounds), S in registers with
 // Phi^-1 in shared memory, both in shared memory; FP64 dot accumulation with
@@ -87,7 +89,8 @@
 #define GBDPCG_VARIANTS_F2_RPT2(NP)                                                           \
     out[c++] = GBDPCG_VARIANT(float, ::gbdpcg::f2acc, NP, false, ST_REG_S, 2);                \
     out[c++] = GBDPCG_VARIANT_REC(float, ::gbdpcg::f2acc, NP, false, ST_REG_S, 2);            \
-    out[c++] = GBDPCG_VARIANT_RF_ACC(NP, ST_REG_S, 2, ::gbdpcg::f2acc);
+    out[c++] = GBDPCG_VARIANT_RF_ACC(NP, ST_REG_S, 2, ::gbdpcg::f2acc);                       \
+    out[c++] = GBDPCG_VARIANT_RF_ACC(NP, ST_TMEM, 2, ::gbdpcg::f2acc);
 // Hybrid storage (sub-diagonal and diagonal S blocks in registers, the
 // super-diagonal block and Phi^-1 in shared memory), standard and recurrence forms.
 #define GBDPCG_VARIANTS_HYB(NP)                                                               \
