@@ -211,6 +211,22 @@ __device__ __forceinline__ void smem_block(const T *col, uint32_t R, const T *x,
 #pragma unroll
     for (int q = 0; q < RPT; ++q) a[q] = acc[q][b];
     uint32_t j = 0;
+    if (n == (uint32_t)NP) {
+        // a full block: no column tests, so the columns are unrolled and their
+        // loads overlap (the row stride is made opaque, or the columns'
+        // addresses, invariant in the PCG loop, would be kept across it and
+        // spilled).  One n=14 N=128 system with a cbtd Phi^-1, both matrices in
+        // shared memory, C 8: 119 -> 86 us; 1024 forward + adjoint pairs of n=14
+        // N=64 with split rows 1796 -> 1758 us.  With column tests instead, for
+        // every n, it was slower than the loop (174 us): a branch a column.
+        asm volatile("" : "+r"(R));
+        T xv[NP];
+        lds_row<T, NP>(xv, x);
+        const T *c = col;
+#pragma unroll
+        for (int u = 0; u < NP; ++u, c += R) smem_col<T, NP, RPT>(c, 0, 0, xv[u], a);
+        j = n;
+    }
 #pragma unroll 2
     for (; j + VW <= n; j += VW) {
         T xv[VW];
