@@ -286,23 +286,34 @@ bool plain_fits(Registry *reg, bool f64, uint32_t n, uint32_t N) {
     return (int64_t)per_sm * reg->sm_count >= (int64_t)N;
 }
 
-// CTAs of a shape that one SM holds at once: its registers (64K in four
-// sub-partitions, whole warps of a multiple of 8 registers a thread) and its
-// shared memory.
+// CTAs of a shape that one SM holds at once: its registers (16K in each of four
+// sub-partitions, a multiple of 8 a thread) and its shared memory.
 uint32_t ctas_per_sm(const Shape &s) {
-    const uint32_t regs = (uint32_t)(s.vi->regs + 7) / 8 * 8, warps = (s.threads / 32 + 3) / 4 * 4;
-    const uint32_t by_regs = 65536u / (regs * 32u * warps);
+    const uint32_t regs = (uint32_t)(s.vi->regs + 7) / 8 * 8;
+    const uint32_t by_regs = 4u * (16384u / (regs * 32u)) / (s.threads / 32);
     const size_t smem = s.vi->v.smem_bytes(s.K, s.C, s.threads / 32) + 1024;
     return std::min<uint32_t>(by_regs, (uint32_t)(228u * 1024u / smem));
 }
 
-// Tensor-memory rows against the storage the preference order finds, for
-// batches: a tensor-memory CTA has its SM to itself, so it pays where the
-// other storage's CTA would have it to itself too (its registers fit the SM
-// once), and not where several of those would share the SM.  Refinement,
-// measured: 256 x n=24 N=256 with C 8 against 16, 91 against 181 ms; 64 x n=24
-// N=64 5.6 / 8.7; 200 x n=14 N=100 16.7 / 19.3; 32 x n=14 N=32 3.74 / 3.95;
-// on the other side 256 x n=8 N=32 (three CTAs of split rows an SM) 4.7 / 3.6.
+// Tensor-memory rows t against the storage s that the preference order finds,
+// for batches with a compact Phi^-1: a tensor-memory CTA has its SM to itself,
+// so it pays where it takes no more of the SMs than the other storage does
+// (t.C CTAs of a whole SM against s.C CTAs, ctas_per_sm(s) of them an SM), and
+// not where several of those would share one.  Measured, us, tensor memory /
+// split rows, 1200 systems of one size: n=14 N=36 298 / 397, N=27 (two split
+// CTAs an SM) 274 / 217; n=24 N=16 304 / 365, N=10 (two) 238 / 175; n=12 N=42
+// 285 / 324, N=32 (two) 263 / 170; n=8 N=96 347 / 429, N=64 (two) 257 / 205;
+// n=6 N=128 358 / 502, N=85 (two) 271 / 239; n=24 N=64, C 2 against 4,
+// 516 / 1046 for 600.  When all of a plan's systems run at once (`one_wave`)
+// every SM holds at most one CTA either way and tensor memory's shorter pass
+// wins everywhere: 152 systems of n=14 N=11 33 / 44, n=6 N=64 42 / 61.
+// Refinement: 256 x n=24 N=256 with C 8 against 16, 91 against 181 ms; 64 x
+// n=24 N=64 5.6 / 8.7; 200 x n=14 N=100 16.7 / 19.3; 256 x n=8 N=32 (three
+// split CTAs an SM) 4.7 / 3.6.
+bool tmem_pays(const Shape &t, const Shape &s, bool one_wave) {
+    return t.C * ctas_per_sm(s) <= s.C || (one_wave && t.C <= s.C);
+}
+
 //
 // c_pref > 1 (lone systems, cluster size not pinned): clusters from c_pref up
 // are tried first, then the smallest that fits.  `lone`: a single system
@@ -314,7 +325,7 @@ uint32_t ctas_per_sm(const Shape &s) {
 int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layout,
                  const gbdpcg_config &cfg, Shape *out, bool refine = false,
                  const TuneChoice *tuned = nullptr, uint32_t c_pref = 1, bool lone = false,
-                 bool fa = false) {
+                 bool fa = false, bool one_wave = false) {
     Shape s;
     const int np = np_for(n);
     if (refine) {
@@ -388,9 +399,19 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
                 return GBDPCG_SUCCESS;
             }
             if (!fit(pf, from, &s)) continue;
-            if (refine && cfg.storage == GBDPCG_STORAGE_AUTO && ctas_per_sm(s) < 2) {
+            // (a lone FP32 system has tried tensor memory first)
+            if (cfg.storage == GBDPCG_STORAGE_AUTO && !ptri && (refine || (!lone && !f64))) {
                 Shape t;
-                if (fit(Pref{4, 2}, from, &t) && t.C <= s.C) s = t;
+                if (fit(Pref{4, 2}, from, &t) && tmem_pays(t, s, one_wave && !refine)) {
+                    // three CTAs at most three quarters full: four, with shorter
+                    // passes (n=24 N=72: 45 against 52 us for one system, 911
+                    // against 857 for 600 of them)
+                    Shape t4;
+                    if (!refine && t.C == 3 && t.K * n * 4 <= (uint32_t)t.vi->max_threads * 2 * 3 && s.C >= 4 &&
+                        fit(Pref{4, 2}, 4, &t4) && t4.C == 4)
+                        t = t4;
+                    s = t;
+                }
             }
             *out = s;
             return GBDPCG_SUCCESS;
@@ -1113,6 +1134,15 @@ int plan_create_impl(gbdpcg_handle_t h, int dtype, const gbdpcg_system *systems,
     // tuned shapes apply unless the config pins the cluster or CTA size
     const bool use_table = !cfg->cluster_size && !cfg->max_threads;
     std::unique_lock<std::mutex> tune_lock(h->tune_mu);
+    // whether all systems run at once with a whole SM for each of their CTAs
+    bool one_wave = count <= (uint32_t)h->reg->sm_count;
+    for (uint32_t i = 0, ctas = 0; i < count && one_wave; ++i) {
+        Shape sh;
+        one_wave = systems[i].n != 0 && systems[i].N != 0 &&
+                   choose_shape(h->reg, p->f64, systems[i].n, systems[i].N, pinv_layout, *cfg, &sh, p->refine, nullptr,
+                                1, false, fa != nullptr, true) == GBDPCG_SUCCESS &&
+                   !sh.plain && (ctas += sh.C) <= (uint32_t)h->reg->sm_count;
+    }
     for (uint32_t i = 0; i < count; ++i) {
         const gbdpcg_system &s = systems[i];
         if (!s.S || !s.Pinv || !s.gamma || !s.lambda || s.n == 0 || s.N == 0)
@@ -1152,7 +1182,8 @@ int plan_create_impl(gbdpcg_handle_t h, int dtype, const gbdpcg_system *systems,
                 tc = &tcv;
             }
         }
-        rc = choose_shape(h->reg, p->f64, s.n, s.N, pinv_layout, *cfg, &sh, p->refine, tc, 1, false, fa != nullptr);
+        rc = choose_shape(h->reg, p->f64, s.n, s.N, pinv_layout, *cfg, &sh, p->refine, tc, 1, false, fa != nullptr,
+                          one_wave);
         if (rc) return rc;
         if (fa && (sh.plain || streamed(sh.vi->v.st)))
             return fail(GBDPCG_ERR_UNSUPPORTED, "a forward + adjoint pair needs the rows on chip (system " +
