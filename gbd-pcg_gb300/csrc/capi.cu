@@ -67,6 +67,8 @@ struct VariantInfo {
 
 struct Registry {
     std::vector<VariantInfo> list;
+    std::vector<GridVariant> grid;  // whole-GPU kernels of one system
+    bool cooperative = false;       // cooperative launches and memory pools
     int max_smem_optin = 0;
     int sm_count = 0;
     // the GPU reads pageable host memory through the host's page tables
@@ -116,6 +118,15 @@ int get_registry(int device, Registry **out) {
             reg->list.push_back(vi);
         }
     }
+    GridVariant gbuf[kMaxGridVariants];
+    for (auto fn : {variants_grid_small, variants_grid_large}) {
+        const int c = fn(gbuf);
+        reg->grid.insert(reg->grid.end(), gbuf, gbuf + c);
+    }
+    int coop = 0, pools = 0;
+    GB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+    GB_CUDA(cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, device));
+    reg->cooperative = coop != 0 && pools != 0;
     GB_CUDA(cudaDeviceGetAttribute(&reg->max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                    device));
     GB_CUDA(cudaDeviceGetAttribute(&reg->sm_count, cudaDevAttrMultiProcessorCount, device));
@@ -449,6 +460,14 @@ struct gbdpcg_handle_s {
     bool last_f64 = false;
     std::mutex tune_mu;  // guards `tune`
     std::map<TuneKey, TuneChoice> tune;
+    // mailboxes of the whole-GPU kernel: one stream-ordered allocation a call
+    // (calls on several streams overlap), from a pool that keeps what calls in
+    // flight together have needed and is given back with the handle
+    std::mutex pool_mu;
+    cudaMemPool_t pool = nullptr;
+    ~gbdpcg_handle_s() {
+        if (pool) cudaMemPoolDestroy(pool);
+    }
 };
 
 namespace {
@@ -591,6 +610,93 @@ int max_active_clusters(const Shape &sh, size_t smem, int *out) {
     return GBDPCG_SUCCESS;
 }
 
+// Whether a lone system goes to the whole-GPU kernel (pcg_grid.cuh): when no
+// on-chip storage of a cluster holds its rows, so that its shape is streamed
+// rows on 16 SMs or the plain algorithm.  Two exchanges over the GPU cost about
+// 4.5 us an iteration (a cluster's reductions under 1 us), so as long as the
+// rows are on a cluster's chips that is faster; past them it never is.
+// Measured, us, streamed or plain / whole GPU: FP32 compact Phi^-1 n=14 N=1500
+// 675 / 198, N=8192 2150 / 240, N=20000 5916 / 445, n=24 N=700 1172 / 189, n=6
+// N=5000 460 / 216; cbtd n=14 N=700 767 / 205, n=24 N=300 562 / 202; FP64
+// n=14 N=440 674 / 573, n=24 N=200 654 / 416, cbtd n=24 N=100 650 / 500.  On
+// chip / whole GPU: FP32 n=14 N=1100 92 / 186, cbtd N=512 163 / 191; FP64 n=14
+// N=256 298 / 382, cbtd N=128 339 / 406.
+bool grid_pays(const Shape &sh, const SysDesc &d, const gbdpcg_config &cfg, bool refine) {
+    return !refine && cfg.algorithm == GBDPCG_ALGO_AUTO && cfg.storage == GBDPCG_STORAGE_AUTO && !cfg.cluster_size &&
+           !cfg.max_threads && cfg.dot_precision == GBDPCG_DOT_NATIVE && !(d.flags & SYS_ADJOINT) &&
+           (sh.plain || streamed(sh.vi->v.st));
+}
+
+// Solves `d` on the whole GPU; *done stays false where the launch does not apply
+// (a shape it does not hold, a stream that is being captured, CTAs that cannot
+// all be resident): the caller then takes another kernel.
+int solve_grid(gbdpcg_handle_s *h, bool f64, const SysDesc &d, uint32_t layout, SysResult *d_res, cudaStream_t stream,
+               bool *done) {
+    *done = false;
+    const Registry *reg = h->reg;
+    const int np = np_for(d.n);
+    if (!reg->cooperative || np == 0 || reg->sm_count <= 0) return GBDPCG_SUCCESS;
+    const uint32_t sms = std::min<uint32_t>((uint32_t)reg->sm_count, kGridMaxCtas);
+    const uint32_t K = (d.N + sms - 1) / sms, C = (d.N + K - 1) / K, rows = K * d.n;
+    const GridVariant *gv = nullptr;
+    for (const GridVariant &v : reg->grid)
+        if (v.f64 == (int)f64 && v.np == np && v.ptri == (int)(layout == GBDPCG_PINV_CBTD) &&
+            rows <= (uint32_t)(v.g * v.max_threads)) {
+            gv = &v;
+            break;
+        }
+    if (!gv) return GBDPCG_SUCCESS;
+    // at least four warps: two that add the values, two that receive the halos
+    const uint32_t threads = std::max<uint32_t>(128, ((rows + gv->g - 1) / gv->g + 31) / 32 * 32);
+    const size_t smem = gv->smem_bytes(K, C, threads / 32);
+    if (smem > (size_t)reg->max_smem_optin) return GBDPCG_SUCCESS;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return GBDPCG_SUCCESS;
+    }
+    {
+        std::lock_guard<std::mutex> lk(h->pool_mu);
+        if (!h->pool) {
+            cudaMemPoolProps props;
+            memset(&props, 0, sizeof(props));
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = h->device;
+            GB_CUDA(cudaMemPoolCreate(&h->pool, &props));
+            uint64_t keep = UINT64_MAX;
+            GB_CUDA(cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        }
+    }
+    if (smem > 48 * 1024)
+        GB_CUDA(cudaFuncSetAttribute(gv->func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t sums = (size_t)2 * kGridWords * C * C * 8, halos = (size_t)2 * C * 2 * 2 * np * 8;
+    void *mail = nullptr;
+    if (cudaMallocFromPoolAsync(&mail, sums + halos, h->pool, stream) != cudaSuccess) {
+        cudaGetLastError();
+        return GBDPCG_SUCCESS;
+    }
+    GridParams gp;
+    memset(&gp, 0, sizeof(gp));
+    gp.one = d;
+    gp.result = d_res;
+    gp.sums = static_cast<uint64_t *>(mail);
+    gp.halos = gp.sums + sums / 8;
+    gp.kmax = K;
+    void *args[] = {&gp};
+    cudaError_t e = cudaMemsetAsync(mail, 0, sums + halos, stream);
+    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(gv->func, dim3(C), dim3(threads), args, smem, stream);
+    const cudaError_t ef = cudaFreeAsync(mail, stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return GBDPCG_SUCCESS;
+    }
+    GB_CUDA(e);
+    GB_CUDA(ef);
+    *done = true;
+    return GBDPCG_SUCCESS;
+}
+
 // One system, device pointers; result left in h->d_last.
 int solve_one(gbdpcg_handle_s *h, bool f64, const SysDesc &d0, const gbdpcg_config &cfg,
               uint32_t layout, cudaStream_t stream, bool refine = false) {
@@ -602,6 +708,16 @@ int solve_one(gbdpcg_handle_s *h, bool f64, const SysDesc &d0, const gbdpcg_conf
     rc = choose_shape(h->reg, f64, d.n, d.N, layout, cfg, &sh, refine, nullptr,
                       lone_cluster_pref(f64 && !refine, d.N), true);
     if (rc) return rc;
+    if (grid_pays(sh, d, cfg, refine)) {
+        bool done = false;
+        rc = solve_grid(h, f64, d, layout, d_res, stream, &done);
+        if (rc) return rc;
+        if (done) {
+            h->d_last = d_res;
+            h->last_stream = stream;
+            return GBDPCG_SUCCESS;
+        }
+    }
     h->d_last = d_res;
     h->last_stream = stream;
     if (sh.plain) {
@@ -1027,7 +1143,17 @@ static int solve_host(bool f64, const void *S, const void *P, const void *g, voi
     // copies (GBDPCG_HOST_STAGING=1 forces the copies).  The results are the
     // same bits either way.
     const char *stage_env = getenv("GBDPCG_HOST_STAGING");
-    const bool direct = h->reg->host_direct && !(stage_env && stage_env[0] == '1');
+    bool direct = h->reg->host_direct && !(stage_env && stage_env[0] == '1');
+    // (no system below a MiB of S goes to a kernel that reads its rows in every
+    // pass; those that do are staged, or every pass would read host memory)
+    if (direct && mat >= ((size_t)1 << 20)) {
+        Shape sh;
+        SysDesc d = make_desc(S, P, g, l, l, n, N, c, build_layout, 0);
+        if (choose_shape(h->reg, f64, n, N, build_layout, c, &sh, false, nullptr, lone_cluster_pref(f64, N), true) ==
+                GBDPCG_SUCCESS &&
+            np_for(n) && grid_pays(sh, d, c, false))
+            direct = false;
+    }
     char *dS, *dP, *dg, *dl;
     if (direct) {
         if (!P) {

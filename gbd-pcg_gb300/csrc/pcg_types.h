@@ -92,4 +92,17 @@ struct LaunchParams {
     SysDesc one;
 };
 
+// Parameters of the whole-GPU kernel of one long system (pcg_grid.cuh).  The
+// mailboxes are zero at the launch.
+struct GridParams {
+    SysDesc one;
+    SysResult *result;
+    uint64_t *sums;   // [2][C receivers][kGridWords][C senders] mailboxes of the reduced values
+    uint64_t *halos;  // [2][C][2 sides][2 NP] mailboxes of the boundary values
+    uint32_t kmax;    // knots per CTA
+    uint32_t pad_;
+};
+constexpr uint32_t kGridWords = 2 * 2;    // two values of up to two 32-bit words
+constexpr uint32_t kGridMaxCtas = 160;    // CTAs whose words a warp polls (5 a lane)
+
 }  // namespace gbdpcg

@@ -48,6 +48,18 @@ int variants_fa_np24(KernelVariant *out);
 int variants_fa_np32(KernelVariant *out);
 int variants_stream_large(KernelVariant *out);  // streamed rows, NP 16..32
 
+// Kernels of one system over the whole GPU (pcg_grid.cuh), native accumulation.
+struct GridVariant {
+    int f64, np, ptri;
+    int g;            // rows per thread
+    int max_threads;
+    const void *func;
+    size_t (*smem_bytes)(uint32_t kmax, uint32_t C, uint32_t nwarps);
+};
+constexpr int kMaxGridVariants = 64;
+int variants_grid_small(GridVariant *out);  // NP 6..14
+int variants_grid_large(GridVariant *out);  // NP 16..32
+
 const void *plain_kernel_ptr(bool f64);
 size_t plain_smem_bytes(bool f64, uint32_t n, uint32_t N);
 
