@@ -33,7 +33,8 @@
 namespace gbdpcg {
 cudaError_t launch_block_jacobi(int kind, const SysDesc *d_descs, const uint64_t *d_prefix,
                                 uint32_t nsys, uint64_t total_knots, int tri_layout,
-                                cudaStream_t stream, const SysDesc *one = nullptr);
+                                cudaStream_t stream, const SysDesc *one, const JacobiClasses *cls);
+int jacobi_class(uint32_t n);  // block-size class of the builder, 0..4 (-1: n > 32)
 }
 
 using namespace gbdpcg;
@@ -239,14 +240,21 @@ std::vector<Pref> storage_prefs(bool f64, bool ptri, uint32_t storage) {
                 : std::vector<Pref>{{1, 2}, {0, 1}, {1, 1}, {2, 1}, {3, 2}, {3, 1}, {5, 2}, {5, 1}};
 }
 
+// Whether a kernel with rpt rows a thread holds blocks of size n: even n always;
+// odd n with an empty last row in the standard and recurrence forms on chip (the
+// single-reduction, refinement and streamed kernels have no such row).
+bool rows_pair(uint32_t n, int st, int rpt, int alg) {
+    return n % (uint32_t)rpt == 0 || ((alg == 0 || alg == 3) && !streamed(st));
+}
+
 // A tuned shape for one system, if its variant exists and holds the system.
 bool tuned_shape(Registry *reg, bool f64, int acc, int np, bool ptri, uint32_t n, uint32_t N,
                  const TuneChoice &tc, Shape *out, bool fa = false) {
-    if (tc.rpt < 1 || n % tc.rpt || tc.C < 1 || tc.C > 16 || tc.threads == 0 || tc.threads % 32) return false;
+    if (tc.rpt < 1 || !rows_pair(n, tc.st, tc.rpt, tc.alg) || tc.C < 1 || tc.C > 16 || tc.threads == 0 || tc.threads % 32) return false;
     VariantInfo *vi = find_variant(reg, f64, acc, np, ptri, tc.st, tc.rpt, tc.alg, fa);
     if (!vi) return false;
     const uint32_t K = (N + tc.C - 1) / tc.C;
-    const uint32_t thr = (K * n + tc.rpt - 1) / tc.rpt;
+    const uint32_t thr = K * ((n + tc.rpt - 1) / tc.rpt);
     if ((!streamed(tc.st) && thr > tc.threads) || tc.threads > (uint32_t)vi->max_threads) return false;
     if (vi->v.smem_bytes(K, tc.C, tc.threads / 32) > (size_t)reg->max_smem_optin) return false;
     out->vi = vi;
@@ -372,7 +380,7 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
         prefs.insert(prefs.begin(), Pref{4, 2});
     // the first cluster size from `from` up at which storage pf holds the system
     auto fit = [&](const Pref &pf, uint32_t from, Shape *o) -> bool {
-        if (pf.rpt > 1 && (n % pf.rpt) != 0) return false;
+        if (!rows_pair(n, pf.st, pf.rpt, alg)) return false;
         VariantInfo *vi = find_variant(reg, f64 && !refine, acc, np, ptri, pf.st, pf.rpt, alg, fa);
         if (!vi) return false;
         uint32_t cap = cfg.max_threads ? cfg.max_threads : (uint32_t)vi->max_threads;
@@ -382,7 +390,7 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
         for (uint32_t C = c_lo; C <= c_hi; ++C) {
             if (C > 8 && (C & (C - 1))) continue;  // large clusters: powers of two only
             const uint32_t K = (N + C - 1) / C;
-            const uint32_t thr = (K * n + pf.rpt - 1) / pf.rpt;
+            const uint32_t thr = K * ((n + pf.rpt - 1) / pf.rpt);
             if (thr > cap && !streamed(pf.st)) continue;
             // CTA sizes are rounded to 64 threads so that systems of similar
             // size share a launch (streamed rows: up to the cap, in row groups)
@@ -402,7 +410,7 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
     };
     for (uint32_t from : {first_lo, 1u}) {
         for (const Pref &pf : prefs) {
-            if (pf.rpt > 1 && (n % pf.rpt) != 0) continue;
+            if (!rows_pair(n, pf.st, pf.rpt, alg)) continue;
             if (streamed(pf.st) && lone && ptri && cfg.storage == GBDPCG_STORAGE_AUTO &&
                 cfg.algorithm == GBDPCG_ALGO_AUTO && cfg.cluster_size == 0 && plain_fits(reg, f64, n, N)) {
                 s.plain = true;
@@ -759,6 +767,7 @@ struct gbdpcg_plan_s {
     DevBuf d_descs, d_order, d_queues, d_results, d_prefix;
     DevBuf plain_scratch;
     uint64_t total_knots = 0;
+    JacobiClasses jacobi;  // (its arrays behind the knot prefix)
     std::vector<cudaStream_t> streams;
     std::vector<cudaEvent_t> events;
     cudaGraph_t graph = nullptr;
@@ -1056,7 +1065,7 @@ static int block_jacobi(gbdpcg_handle_t h, int kind, const void *S, void *P, uin
     d.P = P;
     d.n = n;
     d.N = N;
-    GB_CUDA(launch_block_jacobi(kind, nullptr, nullptr, 1, N, layout == GBDPCG_PINV_CBTD, stream, &d));
+    GB_CUDA(launch_block_jacobi(kind, nullptr, nullptr, 1, N, layout == GBDPCG_PINV_CBTD, stream, &d, nullptr));
     return GBDPCG_SUCCESS;
 }
 
@@ -1334,9 +1343,28 @@ int plan_create_impl(gbdpcg_handle_t h, int dtype, const gbdpcg_system *systems,
     tune_lock.unlock();
     if ((rc = p->d_descs.ensure(sizeof(SysDesc) * count))) return rc;
     if ((rc = p->d_results.ensure(sizeof(SysResult) * p->nresults))) return rc;
-    if ((rc = p->d_prefix.ensure(sizeof(uint64_t) * count))) return rc;
+    // knots before each system; by class: the same, and the systems' indices
+    if ((rc = p->d_prefix.ensure((2 * sizeof(uint64_t) + sizeof(uint32_t)) * count))) return rc;
+    prefix.resize(2 * (size_t)count + (count + 1) / 2);
+    uint64_t *cprefix = prefix.data() + count;
+    std::vector<uint32_t> csys(count);
+    memset(&p->jacobi, 0, sizeof(p->jacobi));
+    for (int c = 0, at = 0; c < 5; ++c) {
+        p->jacobi.first[c] = (uint32_t)at;
+        for (uint32_t i = 0; i < count; ++i) {
+            if (jacobi_class(p->descs[i].n) != c) continue;
+            csys[at] = i;
+            cprefix[at++] = p->jacobi.knots[c];
+            p->jacobi.knots[c] += p->descs[i].N;
+        }
+        p->jacobi.count[c] = (uint32_t)at - p->jacobi.first[c];
+    }
+    memcpy(prefix.data() + 2 * (size_t)count, csys.data(), sizeof(uint32_t) * count);
+    p->jacobi.prefix = p->d_prefix.as<uint64_t>() + count;
+    p->jacobi.sys = reinterpret_cast<const uint32_t *>(p->d_prefix.as<uint64_t>() + 2 * (size_t)count);
     GB_CUDA(cudaMemcpy(p->d_descs.p, p->descs.data(), sizeof(SysDesc) * count, cudaMemcpyHostToDevice));
-    GB_CUDA(cudaMemcpy(p->d_prefix.p, prefix.data(), sizeof(uint64_t) * count, cudaMemcpyHostToDevice));
+    GB_CUDA(cudaMemcpy(p->d_prefix.p, prefix.data(), (2 * sizeof(uint64_t) + sizeof(uint32_t)) * count,
+                       cudaMemcpyHostToDevice));
     GB_CUDA(cudaMemset(p->d_results.p, 0, sizeof(SysResult) * p->nresults));
     if ((rc = plan_layout(p.get()))) return rc;
     const size_t nc = p->classes.size();
@@ -1683,7 +1711,7 @@ int gbdpcg_plan_build_block_jacobi(gbdpcg_plan_t p, gbdpcg_stream_t stream) {
     HandleScope scope(p->h->device);
     GB_CUDA(launch_block_jacobi(p->refine ? 2 : (p->f64 ? 1 : 0), p->d_descs.as<SysDesc>(), p->d_prefix.as<uint64_t>(),
                                 p->count, p->total_knots, p->layout == GBDPCG_PINV_CBTD,
-                                (cudaStream_t)stream));
+                                (cudaStream_t)stream, nullptr, &p->jacobi));
     return GBDPCG_SUCCESS;
 }
 
@@ -1841,7 +1869,7 @@ std::vector<Candidate> tune_candidates(gbdpcg_plan_s *p, const PlanClass &base,
         if (v.fa != (int)p->fused) continue;  // pairs run on the variants built for them
         if (want_st >= 0 && v.st != want_st) continue;
         bool rows_ok = true;
-        for (uint32_t i : items) rows_ok &= p->descs[i].n % v.rpt == 0;
+        for (uint32_t i : items) rows_ok &= rows_pair(p->descs[i].n, v.st, v.rpt, v.alg);
         if (!rows_ok) continue;
         uint32_t cap = std::min<uint32_t>((uint32_t)vi.max_threads,
                                           p->cfg.max_threads ? p->cfg.max_threads : 1024u);
@@ -1854,7 +1882,7 @@ std::vector<Candidate> tune_candidates(gbdpcg_plan_s *p, const PlanClass &base,
                 const uint32_t K = (N + C - 1) / C;
                 ok &= N > (C - 1) * K;  // every CTA of the cluster owns a knot
                 kmax = std::max(kmax, K);
-                thr = std::max(thr, (K * n + v.rpt - 1) / v.rpt);
+                thr = std::max(thr, K * ((n + v.rpt - 1) / v.rpt));
             }
             uint32_t threads = (thr + 31) / 32 * 32;
             if (streamed(v.st)) threads = std::min(threads, cap / 32 * 32);  // row groups beyond the cap

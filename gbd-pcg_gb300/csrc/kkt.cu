@@ -71,167 +71,270 @@ struct Vec16<double> {
     }
 };
 
-// Shared-memory layout of one knot for the formation: Mt[l][r] = M[r][l] with
+// Shared-memory layout of one warp for the formation: Mt[l][r] = M[r][l] with
 // M = [A_k | B_k] (n x (n + m)), i.e. row l of Mt is column l of A_k (l < n)
-// or of B_k, contiguous in global memory, so it loads coalesced with no
-// transpose; rows are NP + 4 elements (a 16-byte multiple), rows n..NP-1 zero.
+// or of B_k, contiguous in global memory; rows are NP + 4 elements (a 16-byte
+// multiple), rows n..NP-1 zero.  X, the Gram product, takes Mt's place.  d, d w
+// (L = n + m each) and Qi_{k+1} follow, then (with the fused inverse) the
+// symmetrised S_kk of every knot the warp inverts at once, Y[c][r] with rows of
+// NP + 4, and the scratch of the inverse.
 template <int NP>
 __host__ __device__ constexpr uint32_t schur_ldt() { return NP + 4; }
+// knots a warp inverts at once
+template <int NP>
+__host__ __device__ constexpr uint32_t schur_knots() { return 32 / gbdpcg::gj_lanes(NP); }
 
-// per-warp elements: Mt (L rows) + d (L) + w (L) + Qi_{k+1} (32) + two pivot
-// rows of the fused block-Jacobi inverse (32 each), L = n + m
-__host__ __device__ inline uint32_t schur_warp_elems(uint32_t L, uint32_t ldt) {
-    return (L * ldt + 2 * ((L + 3) & ~3u) + 96);
+template <int NP>
+__host__ __device__ inline uint32_t schur_mt_elems(uint32_t L) {
+    const uint32_t mt = L * schur_ldt<NP>(), x = (NP * (NP + 1) + 3) & ~3u;
+    return mt > x ? mt : x;
+}
+template <int NP, bool PINV>
+__host__ __device__ inline uint32_t schur_warp_elems(uint32_t L) {
+    return schur_mt_elems<NP>(L) + 2 * ((L + 3) & ~3u) + 32 +
+           (PINV ? schur_knots<NP>() * NP * schur_ldt<NP>() + gbdpcg::kGjElems : 0);
 }
 
-// Asynchronous copy of one element global -> shared (cp.async, no registers,
-// nothing waits until cp_async_wait_all); valid = false writes a zero instead.
-template <typename T>
-__device__ __forceinline__ void cp_async_elem(T *smem, const T *gmem, bool valid) {
-    const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-    const uint32_t bytes = valid ? (uint32_t)sizeof(T) : 0u;
-    if constexpr (sizeof(T) == 4)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+// Asynchronous copy of VW consecutive elements global -> shared (cp.async, no
+// registers, nothing waits until cp_async_wait_all).
+template <typename T, int VW>
+__device__ __forceinline__ void cp_async_vec(T *smem, const T *gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem),
+                 "n"((int)(VW * sizeof(T)))
+                 : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// loads TR consecutive elements starting at an 8-byte-aligned float address
-// (pairs) or any double address
-template <typename T, int TR>
-__device__ __forceinline__ void load_run(const T *p, T (&v)[TR]) {
-    if constexpr (sizeof(T) == 4 && TR % 2 == 0) {
-#pragma unroll
-        for (int t = 0; t < TR; t += 2) {
-            const float2 x = *reinterpret_cast<const float2 *>(p + t);
-            v[t] = x.x;
-            v[t + 1] = x.y;
-        }
+// VW consecutive elements as one access (VW sizeof(T) bytes, 16 at most).
+template <typename T, int VW>
+__device__ __forceinline__ void store_vec(T *p, const T (&v)[VW]) {
+    if constexpr (sizeof(T) * VW == 16 && sizeof(T) == 4)
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else if constexpr (sizeof(T) * VW == 16)
+        *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+    else if constexpr (sizeof(T) * VW == 8 && VW == 2)
+        *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+    else
+        p[0] = v[0];
+}
+template <typename T, int VW>
+__device__ __forceinline__ void load_vec(const T *p, T (&v)[VW]) {
+    if constexpr (sizeof(T) * VW == 16 && sizeof(T) == 4) {
+        const float4 t = *reinterpret_cast<const float4 *>(p);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (sizeof(T) * VW == 16) {
+        const double2 t = *reinterpret_cast<const double2 *>(p);
+        v[0] = t.x; v[1] = t.y;
+    } else if constexpr (sizeof(T) * VW == 8 && VW == 2) {
+        const float2 t = *reinterpret_cast<const float2 *>(p);
+        v[0] = t.x; v[1] = t.y;
     } else {
-#pragma unroll
-        for (int t = 0; t < TR; ++t) v[t] = p[t];
+        v[0] = p[0];
     }
 }
 
-// One warp per knot.  The Gram product S_kk = M diag(d) M^T is a 2D register
-// tile per lane: lanes form a 4 x 8 grid, lane (rg, cg) owns rows
+// The Gram product M diag(d) M^T of the NP-row columns in Mt as a TR x TC tile
+// per lane, rows from r0, columns from c0: acc[t][u] = sum_l fma(M[r0+t][l] d_l,
+// M[c0+u][l], .) in ascending l; FP32 two rows an instruction (fma.rn.f32x2).
+template <typename T, int TR, int TC>
+__device__ __forceinline__ void gram_tile(const T *Mt, uint32_t ldt, const T *dv, uint32_t L, uint32_t r0, uint32_t c0,
+                                          T (&acc)[TR][TC]) {
+    if constexpr (sizeof(T) == 4) {
+        unsigned long long s[TR / 2][TC];
+#pragma unroll
+        for (int t = 0; t < TR / 2; ++t)
+#pragma unroll
+            for (int u = 0; u < TC; ++u) s[t][u] = 0ull;
+        const T *a = Mt + r0, *b = Mt + c0;
+#pragma unroll 2
+        for (uint32_t l = 0; l < L; ++l, a += ldt, b += ldt) {
+            const float d = dv[l];
+            const unsigned long long dd = gbdpcg::pack2(d, d);
+            unsigned long long ad[TR / 2];
+#pragma unroll
+            for (int t = 0; t < TR / 2; ++t)
+                ad[t] = gbdpcg::mul2(*reinterpret_cast<const unsigned long long *>(a + 2 * t), dd);
+#pragma unroll
+            for (int u = 0; u < TC; ++u) {
+                const unsigned long long bb = gbdpcg::pack2(b[u], b[u]);
+#pragma unroll
+                for (int t = 0; t < TR / 2; ++t) s[t][u] = gbdpcg::fma2(ad[t], bb, s[t][u]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < TR / 2; ++t)
+#pragma unroll
+            for (int u = 0; u < TC; ++u) {
+                acc[2 * t][u] = gbdpcg::lo2(s[t][u]);
+                acc[2 * t + 1][u] = gbdpcg::hi2(s[t][u]);
+            }
+    } else {
+#pragma unroll
+        for (int t = 0; t < TR; ++t)
+#pragma unroll
+            for (int u = 0; u < TC; ++u) acc[t][u] = T(0);
+#pragma unroll 2
+        for (uint32_t l = 0; l < L; ++l) {
+            const T d = dv[l];
+            T b[TC];
+#pragma unroll
+            for (int u = 0; u < TC; ++u) b[u] = Mt[l * ldt + c0 + u];
+#pragma unroll
+            for (int t = 0; t < TR; ++t) {
+                const T ad = Mt[l * ldt + r0 + t] * d;
+#pragma unroll
+                for (int u = 0; u < TC; ++u) acc[t][u] += ad * b[u];
+            }
+        }
+    }
+}
+
+// Schur formation: a warp forms kw knots in turn (1; with the fused inverse up to
+// as many as it then inverts at once).  The Gram product S_kk = M diag(d) M^T is a
+// 2D register tile per lane: lanes form a 4 x 8 grid, lane (rg, cg) owns rows
 // rg TR .. rg TR + TR - 1 and columns cg TC .. cg TC + TC - 1 of the NP x NP
-// product (TR = NP / 4, TC = NP / 8), and each column l of M adds a rank-1
-// term: TR + TC shared-memory loads for TR TC FMAs.  Every element is rounded
-// as sum_l fma(M[i][l] d_l, M[j][l], .) in ascending l, then + Qi_{k+1} on the
-// diagonal, and symmetrised as 0.5 (S + S^T) through shared memory.  With
-// PINV the warp then inverts the symmetrised S_kk (rotating Gauss-Jordan, the
-// block-Jacobi builder's own routine and rounding) and writes the compact
-// block-Jacobi Phi^-1, so the preconditioner is built with S and never
-// re-read.
-template <typename T, int NP, int W, bool PINV>
-__global__ void __launch_bounds__(W * 32)
+// product (TR = NP / 4, TC = NP / 8).  It is rounded as in gram_tile, then + Qi_{k+1}
+// on the diagonal, and symmetrised as 0.5 (S + S^T) through shared memory.  With
+// PINV the warp then inverts the symmetrised S_kk (the block-Jacobi builder's own
+// routine and rounding) and writes the compact block-Jacobi Phi^-1, so the
+// preconditioner is built with S and never re-read.
+//
+// VW: elements of one global access (16 bytes where n is a multiple of their
+// number and the arrays are aligned, else 8, else one element).  The blocks are
+// contiguous, so a warp walks them in pieces of VW with one division an access.
+//
+// What bounds it: instruction issue and the shared-memory pipe (n=24, m=12: 5930
+// instructions a knot with one element an access, one row an FMA and a select an
+// element of the inverse; now 4200, the pipe 71% busy).  The register caps keep 28
+// warps on an SM (n=24 with Phi^-1 at 96 registers: 365 us).  Measured, us, before
+// and now, N=65536 FP32: n=24 m=12 212 -> 183, with Phi^-1 382 -> 329; n=14 m=7
+// 114 -> 102, 198 -> 140; n=6 m=3 with Phi^-1 96 -> 56.  FP64 is bound by the FP64
+// pipe (n=14 m=7 N=30000 with Phi^-1 1365 -> 980).
+template <typename T, int NP, int W, bool PINV, int VW>
+__global__ void __launch_bounds__(W * 32, sizeof(T) == 4 ? (NP <= 24 ? 7 : 5) : 6)
     form_schur_kernel(const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ Qd,
                       const T *__restrict__ Rd, const T *__restrict__ q, const T *__restrict__ r,
-                      const T *__restrict__ c, uint32_t n, uint32_t m, uint32_t N, T *__restrict__ S,
+                      const T *__restrict__ c, uint32_t n, uint32_t m, uint32_t N, uint32_t kw, T *__restrict__ S,
                       T *__restrict__ gamma, T *__restrict__ Pinv) {
-    constexpr int TR = NP / 4, TC = NP / 8;
-    constexpr uint32_t ldt = schur_ldt<NP>();
+    constexpr int TR = NP / 4, TC = NP / 8, GL = gbdpcg::gj_lanes(NP);
+    constexpr uint32_t ldt = schur_ldt<NP>(), xs = NP + 1, KW = PINV ? schur_knots<NP>() : 1;
     extern __shared__ __align__(16) unsigned char schur_smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t k = blockIdx.x * W + warp;
-    if (k >= N) return;  // warp-uniform; no CTA barrier below
-    const uint32_t L = n + m, L4 = (L + 3) & ~3u;
-    T *Mt = reinterpret_cast<T *>(schur_smem) + (size_t)warp * schur_warp_elems(L, ldt);
-    T *dv = Mt + L * ldt, *wv = dv + L4, *qn = wv + L4, *s_raw = qn + 32, *s_t = s_raw + 32;
-    const T *Ak = A + (size_t)k * n * n, *Bk = B + (size_t)k * n * m;
-    // every column in flight at once (cp.async); rows n..NP-1 zero-filled
-    for (uint32_t l = 0; l < L; ++l) {
-        const T *src = l < n ? Ak + (size_t)l * n : Bk + (size_t)(l - n) * n;
-        if (lane < (uint32_t)NP) cp_async_elem(Mt + l * ldt + lane, src + (lane < n ? lane : 0u), lane < n);
-    }
-    if (lane < n) {
-        dv[lane] = T(1) / Qd[(size_t)k * n + lane];
-        wv[lane] = q[(size_t)k * n + lane];
-        qn[lane] = T(1) / Qd[(size_t)(k + 1) * n + lane];
-    }
-    if (lane < m) {
-        dv[n + lane] = T(1) / Rd[(size_t)k * m + lane];
-        wv[n + lane] = r[(size_t)k * m + lane];
-    }
-    cp_async_wait_all();
-    __syncwarp();
-    T *Sk = S + (size_t)k * 3 * n * n;
-    // block 0 of row k: S_{k,k-1}, element (i, j) = -Qi_k[j] A_k[i][j]; block 2
-    // of row k-1: S_{k-1,k}, element (i, j) = -Qi_k[i] A_k[j][i] (this warp holds
-    // A_k, so each A_k is read once); the last row's block 2 is padding
-    T *Sup = (k > 0) ? S + (size_t)(k - 1) * 3 * n * n + 2 * (size_t)n * n : nullptr;
-    if (lane < n) {  // column by column, lane = row: coalesced, no index division
-        const uint32_t row = lane;
-        for (uint32_t col = 0; col < n; ++col) {
-            const uint32_t e = col * n + row;
-            Sk[e] = (k > 0) ? -dv[col] * Mt[col * ldt + row] : T(0);
-            if (k > 0) Sup[e] = -dv[row] * Mt[row * ldt + col];
-            if (k + 1 == N) Sk[2 * (size_t)n * n + e] = T(0);
+    const uint32_t k0 = (blockIdx.x * W + warp) * kw;
+    if (k0 >= N) return;  // warp-uniform; no CTA barrier below
+    const uint32_t L = n + m, L4 = (L + 3) & ~3u, nn = n * n;
+    T *Mt = reinterpret_cast<T *>(schur_smem) + (size_t)warp * schur_warp_elems<NP, PINV>(L);
+    T *X = Mt, *dv = Mt + schur_mt_elems<NP>(L), *dw = dv + L4, *qn = dw + L4, *Y = qn + 32, *s = Y + KW * NP * ldt;
+    // pieces of VW elements: n / VW in a column; x / cv = (x magic) >> 16 for x < 2048
+    const uint32_t cv = n / VW, magic = (65536u + cv - 1) / cv;
+    const uint32_t kend = min(k0 + kw, N);
+    for (uint32_t k = k0; k < kend; ++k) {
+        const T *Ak = A + (size_t)k * nn, *Bk = B + (size_t)k * n * m;
+        // every column in flight at once (cp.async)
+        for (uint32_t e = lane; e < L * cv; e += 32) {
+            const uint32_t l = (e * magic) >> 16, p = (e - l * cv) * VW;
+            cp_async_vec<T, VW>(Mt + l * ldt + p, l < n ? Ak + e * VW : Bk + (e - n * cv) * VW);
+        }
+        if (n < (uint32_t)NP)  // rows n..NP-1
+            for (uint32_t l = lane; l < L; l += 32)
+                for (uint32_t p = n; p < (uint32_t)NP; ++p) Mt[l * ldt + p] = T(0);
+        if (lane < n) {
+            const T d = T(1) / Qd[(size_t)k * n + lane];
+            dv[lane] = d;
+            dw[lane] = d * q[(size_t)k * n + lane];
+            qn[lane] = T(1) / Qd[(size_t)(k + 1) * n + lane];
+        }
+        if (lane < m) {
+            const T d = T(1) / Rd[(size_t)k * m + lane];
+            dv[n + lane] = d;
+            dw[n + lane] = d * r[(size_t)k * m + lane];
+        }
+        cp_async_wait_all();
+        __syncwarp();
+        T *Sk = S + (size_t)k * 3 * nn;
+        // block 0 of row k: S_{k,k-1}, element (i, j) = -Qi_k[j] A_k[i][j]; block 2
+        // of row k-1: S_{k-1,k}, element (i, j) = -Qi_k[i] A_k[j][i] (this warp holds
+        // A_k, so each A_k is read once); the last row's block 2 is padding
+        T *Sup = (k > 0) ? S + (size_t)(k - 1) * 3 * nn + 2 * (size_t)nn : nullptr;
+        for (uint32_t e = lane; e < n * cv; e += 32) {
+            const uint32_t col = (e * magic) >> 16, p = (e - col * cv) * VW;
+            T v[VW], w[VW], d[VW];
+            if (k > 0) {
+                load_vec<T, VW>(Mt + col * ldt + p, v);
+                load_vec<T, VW>(dv + p, d);
+#pragma unroll
+                for (int u = 0; u < VW; ++u) {
+                    v[u] = -dv[col] * v[u];
+                    w[u] = -d[u] * Mt[(p + u) * ldt + col];
+                }
+                store_vec<T, VW>(Sup + e * VW, w);
+            } else {
+#pragma unroll
+                for (int u = 0; u < VW; ++u) v[u] = T(0);
+            }
+            store_vec<T, VW>(Sk + e * VW, v);
+            if (k + 1 == N) {
+#pragma unroll
+                for (int u = 0; u < VW; ++u) v[u] = T(0);
+                store_vec<T, VW>(Sk + 2 * (size_t)nn + e * VW, v);
+            }
         }
         // gamma_k = -(c_k + M diag(d) w - Qi_{k+1} q_{k+1})
-        T g = T(0);
-        for (uint32_t l = 0; l < L; ++l) g += Mt[l * ldt + row] * (dv[l] * wv[l]);
-        gamma[(size_t)k * n + row] = -(c[(size_t)k * n + row] + g - qn[row] * q[(size_t)(k + 1) * n + row]);
-    }
-    // the Gram tile
-    const uint32_t rg = lane >> 3, cg = lane & 7, r0 = rg * TR, c0 = cg * TC;
-    T acc[TR][TC];
-#pragma unroll
-    for (int t = 0; t < TR; ++t)
-#pragma unroll
-        for (int u = 0; u < TC; ++u) acc[t][u] = T(0);
-#pragma unroll 2
-    for (uint32_t l = 0; l < L; ++l) {
-        T a[TR], b[TC];
-        load_run<T, TR>(Mt + l * ldt + r0, a);
-#pragma unroll
-        for (int u = 0; u < TC; ++u) b[u] = Mt[l * ldt + c0 + u];
-        const T d = dv[l];
-#pragma unroll
-        for (int t = 0; t < TR; ++t) {
-            const T ad = a[t] * d;
-#pragma unroll
-            for (int u = 0; u < TC; ++u) acc[t][u] += ad * b[u];
+        if (lane < n) {
+            T g = T(0);
+#pragma unroll 4
+            for (uint32_t l = 0; l < L; ++l) g += Mt[l * ldt + lane] * dw[l];
+            gamma[(size_t)k * n + lane] = -(c[(size_t)k * n + lane] + g - qn[lane] * q[(size_t)(k + 1) * n + lane]);
         }
-    }
-    __syncwarp();  // every lane is done with Mt: it now holds S_kk, row stride NP + 1
-    constexpr uint32_t xs = NP + 1;
-    T *X = Mt;
+        const uint32_t r0 = (lane >> 3) * TR, c0 = (lane & 7) * TC;
+        T acc[TR][TC];
+        gram_tile<T, TR, TC>(Mt, ldt, dv, L, r0, c0, acc);
+        __syncwarp();  // every lane is done with Mt: it now holds the product, row stride NP + 1
 #pragma unroll
-    for (int t = 0; t < TR; ++t)
+        for (int t = 0; t < TR; ++t)
 #pragma unroll
-        for (int u = 0; u < TC; ++u) {
-            const uint32_t i = r0 + t, j = c0 + u;
-            if (i < n && j < n) X[i * xs + j] = (i == j) ? acc[t][u] + qn[i] : acc[t][u];
+            for (int u = 0; u < TC; ++u) {
+                const uint32_t i = r0 + t, j = c0 + u;
+                if (i < n && j < n) X[i * xs + j] = (i == j) ? acc[t][u] + qn[i] : acc[t][u];
+            }
+        __syncwarp();
+        // block 1: S_kk symmetrised, kept for the inverse
+        T *Yk = Y + (k - k0) * NP * ldt;
+        for (uint32_t e = lane; e < n * cv; e += 32) {
+            const uint32_t col = (e * magic) >> 16, p = (e - col * cv) * VW;
+            T v[VW];
+#pragma unroll
+            for (int u = 0; u < VW; ++u) v[u] = T(0.5) * (X[(p + u) * xs + col] + X[col * xs + p + u]);
+            store_vec<T, VW>(Sk + nn + e * VW, v);
+            if constexpr (PINV) store_vec<T, VW>(Yk + col * ldt + p, v);
         }
-    __syncwarp();
-    // block 1: S_kk symmetrised
-    if (lane < n) {
-        const uint32_t row = lane;
-        for (uint32_t col = 0; col < n; ++col)
-            Sk[n * n + col * n + row] = T(0.5) * (X[row * xs + col] + X[col * xs + row]);
+        __syncwarp();  // X is free for the next knot's columns, Y complete
     }
     if constexpr (PINV) {
-        // lane r: row r of the symmetrised S_kk (the values just written),
-        // identity beyond n
+        // group g of GL lanes: knot k0 + g; lane rr: row rr of the symmetrised S_kk
+        // (the values just written), identity beyond n
+        const uint32_t g = lane / GL, rr = lane % GL;
+        const bool mine = k0 + g < kend && rr < n;
+        const T *Yg = Y + g * NP * ldt;
         T a[NP];
 #pragma unroll
         for (int cc = 0; cc < NP; ++cc)
-            a[cc] = (lane < n && (uint32_t)cc < n) ? T(0.5) * (X[lane * xs + cc] + X[cc * xs + lane])
-                                                   : ((uint32_t)cc == lane ? T(1) : T(0));
-        gbdpcg::gj_rotate<T, NP>(a, s_raw, s_t, lane);  // ends with a warp sync: X is free
-        if (lane < n) {
+            a[cc] = (mine && (uint32_t)cc < n) ? Yg[cc * ldt + rr] : ((uint32_t)cc == rr ? T(1) : T(0));
+        const T diag = mine ? Yg[rr * ldt + rr] : T(1);
+        T *sg = s + g * 3 * GL;
+        const T h = T(0.5) * gbdpcg::gj_inverse<T, NP, GL>(a, diag, sg, rr);  // ends with a warp sync: Y is free
+        const T *D = sg + 2 * GL;
+        T *Xg = Y + g * NP * ldt;
+        if (rr < (uint32_t)NP) {
 #pragma unroll
-            for (int cc = 0; cc < NP; ++cc)
-                if ((uint32_t)cc < n) X[lane * xs + cc] = a[cc];
+            for (int cc = 0; cc < NP; ++cc) Xg[rr * xs + cc] = a[cc];
         }
         __syncwarp();
-        if (lane < n) {  // symmetrised, compact n^2 per knot, column-major
-            T *Pk = Pinv + (size_t)k * n * n;
-            for (uint32_t col = 0; col < n; ++col)
-                Pk[col * n + lane] = T(0.5) * (X[lane * xs + col] + X[col * xs + lane]);
+        if (mine) {  // symmetrised, compact n^2 per knot, column-major
+            T *Pk = Pinv + (size_t)(k0 + g) * nn;
+#pragma unroll
+            for (int cc = 0; cc < NP; ++cc)
+                if ((uint32_t)cc < n) Pk[cc * n + rr] = gbdpcg::mul_pow2(a[cc] + Xg[cc * xs + rr], h, D[cc]);
         }
     }
 }
@@ -320,19 +423,36 @@ int form_schur(const T *A, const T *B, const T *Qd, const T *Rd, const T *q, con
     int rc = check(p, 9, n, m, N);
     if (rc) return rc;
     constexpr int W = kkt_warps<T>();
+    // elements of an access: what n and the blocks' addresses allow
+    const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(S);
+    constexpr uint32_t V16 = 16 / sizeof(T);
+    const bool v16 = n % V16 == 0 && (at & 15u) == 0, v8 = sizeof(T) == 4 && n % 2 == 0 && (at & 7u) == 0;
     auto go = [&](auto np) -> int {
         constexpr int NP = decltype(np)::value;
-        const size_t smem = (size_t)W * schur_warp_elems(n + m, schur_ldt<NP>()) * sizeof(T);
-        auto launch = [&](auto kern) -> int {
+        auto launch = [&](auto kern, size_t smem, uint32_t knots) -> int {
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) {
                 gbdpcg::set_last_error(std::string("form_schur: ") + cudaGetErrorString(e));
                 return GBDPCG_ERR_CUDA;
             }
-            kern<<<(N + W - 1) / W, W * 32, smem, st>>>(A, B, Qd, Rd, q, r, c, n, m, N, S, gamma, Pinv);
+            // few knots: one a warp, side by side (n=14 N=500: 10.5 us against 11.8
+            // with two in turn); as many as a warp inverts at once from the knots
+            // on that fill the GPU's warps
+            if (N <= 4096) knots = 1;
+            kern<<<(N + W * knots - 1) / (W * knots), W * 32, smem, st>>>(A, B, Qd, Rd, q, r, c, n, m, N, knots, S, gamma,
+                                                                          Pinv);
             return launched("form_schur");
         };
-        return Pinv ? launch(form_schur_kernel<T, NP, W, true>) : launch(form_schur_kernel<T, NP, W, false>);
+        auto width = [&](auto vw) -> int {
+            constexpr int VW = decltype(vw)::value;
+            const size_t w = (size_t)W * sizeof(T);
+            return Pinv ? launch(form_schur_kernel<T, NP, W, true, VW>, w * schur_warp_elems<NP, true>(n + m), schur_knots<NP>())
+                        : launch(form_schur_kernel<T, NP, W, false, VW>, w * schur_warp_elems<NP, false>(n + m), 1);
+        };
+        if (v16) return width(std::integral_constant<int, (int)V16>());
+        if constexpr (sizeof(T) == 4)
+            if (v8) return width(std::integral_constant<int, 2>());
+        return width(std::integral_constant<int, 1>());
     };
     if (n <= 8) return go(std::integral_constant<int, 8>());
     if (n <= 16) return go(std::integral_constant<int, 16>());

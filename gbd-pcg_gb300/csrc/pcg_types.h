@@ -92,6 +92,16 @@ struct LaunchParams {
     SysDesc one;
 };
 
+// A batch by the block-size classes of the block-Jacobi builder (n <= 8, 12, 16,
+// 24, 32): device arrays of the systems' indices and of the knots of the class
+// before each, class c's at [first[c], first[c] + count[c]).
+struct JacobiClasses {
+    const uint32_t *sys;
+    const uint64_t *prefix;
+    uint32_t first[5], count[5];
+    uint64_t knots[5];
+};
+
 // Parameters of the whole-GPU kernel of one long system (pcg_grid.cuh).  The
 // mailboxes are zero at the launch.
 struct GridParams {

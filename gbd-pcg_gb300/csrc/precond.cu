@@ -2,119 +2,341 @@
 //
 // The reference takes Phi^-1 from its caller (include/interface.cuh:24-32) and
 // its documented pcg_solve(S, gamma, lambda, ...) (README.md:42) has no Phi^-1
-// argument; this kernel supplies it.  One warp per knot: lane r holds row r of
-// the diagonal block S_kk (the middle block of the cbtd block row) in
-// registers, padded with the identity to NP x NP (NP in {8, 12, 16, 24, 32},
-// the smallest that holds n), and the warp inverts it by Gauss-Jordan
-// elimination without pivoting (S_kk is symmetric positive definite) in the
-// rotating form: step j pivots on row j and on the row's first register; every
-// row then shifts one column to the left and the column of the inverse being
-// formed enters at the right, so all register indices are compile-time
-// constants while the step loop stays rolled, and after NP steps the columns
-// are back in order.  The pivot row goes through shared memory: lane j stores
-// it, lane c scales its element c, and every lane reads the scaled row back
-// with 16-byte broadcast loads.  A shared-memory transpose symmetrises the
-// inverse, written either as a cbtd block row [0 | S_kk^-1 | 0] or compactly
-// (n^2 per knot, column-major), column by column.  Work item = (system, knot)
-// over a batch; the knot-prefix array maps a warp to its system.  TI: element
-// type of S, TO: of Phi^-1, CT: arithmetic (double S with float Phi^-1 serves
-// the FP32-inner refinement).
+// argument; this kernel supplies it.  The diagonal blocks S_kk (the middle block
+// of a cbtd block row) are inverted in registers, a group of 8, 16 or 32 lanes a
+// block (gauss_jordan.cuh), padded with the identity to NP x NP (NP in {8, 12,
+// 16, 24, 32}, the smallest that holds n).  A shared-memory transpose symmetrises
+// the inverse, written either as a cbtd block row [0 | S_kk^-1 | 0] or compactly
+// (n^2 per knot, column-major), column by column.
+//
+// A warp takes `per` consecutive knots of the batch (the knot-prefix array maps
+// them to systems) and inverts as many at once as their n allows.
+//
+// Two kernels.  FP32 batches with 8192 knots or more of a block-size class take
+// four rows a lane (block_jacobi_quad_kernel): 16 to 4 blocks a warp share the
+// search for their system, the divisions and the barriers.  Everything else takes
+// one row a lane: few knots, because one block then has the shorter chain and
+// runs beside the others (one system of n=14, 60 knots: 6.9 us against 9.1 with
+// two a warp), and FP64, whose pipe (two lanes a clock per SM) bounds it: there
+// two blocks of n <= 16 a warp instead of one halve the instructions (1024
+// systems of n=14, 1634 -> 823 us), and n = 24 gains 2%.
+//
+// Measured, FP32, us, one block a warp with a scaled pivot row / one row a lane /
+// four: 2048 systems of 16 to 128 knots, n=14 302 / 143 / 108, n=6 173 / 57 / 34,
+// n in {6, 12, 14, 24} 317 / 225 / 190; 1024 of n=24 269 / 250 / 181; 512 of n=32
+// 223 / 287 / 181.  What bounds four rows a lane is the fetch of its long
+// straight-line code by two or three warps a scheduler (n=24: 990 instructions a
+// block, issued at 37%).  TI: element type of S, TO: of Phi^-1, CT: arithmetic (double S
+// with float Phi^-1 serves the FP32-inner refinement).
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
+
+#include <type_traits>
 
 #include "gauss_jordan.cuh"
 #include "pcg_types.h"
 
 namespace gbdpcg {
 
-constexpr int kPrecWarps = 4;  // knots per CTA
+constexpr int kPrecWarps = 4;  // warps per CTA
 constexpr int kPrecMaxN = 32;
+// elements of the transposes of a warp's blocks: 32 rows of 33, or two of 16 x 17,
+// or four of 8 x 9
+constexpr int kPrecX = kPrecMaxN * (kPrecMaxN + 1);
 
+// The classes of block sizes: NP = 8, 12, 16, 24, 32; -1 outside.
+__host__ __device__ constexpr int np_class(uint32_t n) {
+    return n == 0 ? -1 : (n <= 8 ? 0 : (n <= 12 ? 1 : (n <= 16 ? 2 : (n <= 24 ? 3 : (n <= (uint32_t)kPrecMaxN ? 4 : -1)))));
+}
+
+// The last s in [0, nsys) with knot_prefix[s] <= gk, by a whole warp: 32 probes a
+// round (three rounds of loads for 32768 systems where a binary search pays 15
+// one after another).
+__device__ __forceinline__ uint32_t find_system(const uint64_t *__restrict__ knot_prefix, uint32_t nsys, uint64_t gk,
+                                                uint32_t lane) {
+    uint32_t lo = 0, len = nsys;
+    while (len > 1) {
+        const uint32_t step = (len + 31) / 32, i = lane * step;
+        const uint32_t below = __popc(__ballot_sync(0xffffffffu, i < len && knot_prefix[lo + i] <= gk));
+        lo += (below - 1) * step;  // (the first probe always holds)
+        len = min(step, len - (below - 1) * step);
+    }
+    return lo;
+}
+
+// Inverts `cnt` blocks of one system at once (cnt <= 32 / GL): block g's S_kk at
+// Sk + g strideS, its row of Phi^-1 at row + g strideP.  Groups from cnt on run on
+// the identity and write nothing.
 template <typename TI, typename TO, typename CT, int NP>
-__device__ __forceinline__ void invert_knot(const TI *Sk, TO *row, uint32_t n, int tri_layout, CT *s_raw, CT *s_t,
-                                            CT *X, uint32_t lane) {
-    // lane r: row r of S_kk (column-major: (r, c) at c*n + r; coalesced over
-    // lanes), identity beyond n
+__device__ __forceinline__ void invert_knots(const TI *Sk, TO *row, uint32_t n, uint32_t cnt, int tri_layout, CT *s, CT *X,
+                                             uint32_t lane) {
+    constexpr int GL = gj_lanes(NP), LD = GL + 1;
+    const uint32_t g = lane / GL, r = lane % GL;
+    const bool mine = g < cnt && r < n;
+    Sk += (size_t)g * 3 * n * n;
+    row += (size_t)g * (tri_layout ? 3 : 1) * n * n;
+    // row r of S_kk (column-major: (r, c) at c*n + r; coalesced over lanes),
+    // identity beyond n
     CT a[NP];
 #pragma unroll
     for (int c = 0; c < NP; ++c)
-        a[c] = (lane < n && (uint32_t)c < n) ? CT(Sk[(size_t)c * n + lane]) : ((uint32_t)c == lane ? CT(1) : CT(0));
-    gj_rotate<CT, NP>(a, s_raw, s_t, lane);
-    // symmetrise through a shared-memory transpose: X[r][c] = inverse (r, c)
-    const uint32_t ld = kPrecMaxN + 1;
-    if (lane < n) {
+        a[c] = (mine && (uint32_t)c < n) ? CT(Sk[(size_t)c * n + r]) : ((uint32_t)c == r ? CT(1) : CT(0));
+    const CT diag = mine ? CT(Sk[(size_t)r * n + r]) : CT(1);
+    s += g * 3 * GL;
+    X += g * GL * LD;
+    const CT h = CT(0.5) * gj_inverse<CT, NP, GL>(a, diag, s, r);  // (lanes without a row: 0, not used)
+    const CT *D = s + 2 * GL;
+    // symmetrise through a shared-memory transpose: X[r][c] = a[c] of lane r
+    if (r < (uint32_t)NP) {
 #pragma unroll
-        for (int c = 0; c < NP; ++c)
-            if ((uint32_t)c < n) X[lane * ld + c] = a[c];
+        for (int c = 0; c < NP; ++c) X[r * LD + c] = a[c];
     }
     __syncwarp();
     // column by column, lane = row: coalesced stores, no index division
     const uint32_t nn = n * n, mid = tri_layout ? nn : 0;
-    if (lane < n) {
-        const uint32_t r = lane;
-        for (uint32_t c = 0; c < n; ++c) {
-            row[mid + c * n + r] = TO(CT(0.5) * (X[r * ld + c] + X[c * ld + r]));
-            if (tri_layout) {
-                row[c * n + r] = TO(0);
-                row[2 * nn + c * n + r] = TO(0);
+    if (mine) {
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+            if ((uint32_t)c < n) {
+                row[mid + c * n + r] = TO(mul_pow2(a[c] + X[c * LD + r], h, D[c]));
+                if (tri_layout) {
+                    row[c * n + r] = TO(0);
+                    row[2 * nn + c * n + r] = TO(0);
+                }
             }
         }
     }
+    __syncwarp();
 }
 
 template <typename TI, typename TO, typename CT>
-__global__ void __launch_bounds__(kPrecWarps * 32)
+__global__ void __launch_bounds__(kPrecWarps * 32, sizeof(CT) == 4 ? 5 : 4)
     block_jacobi_kernel(const SysDesc *__restrict__ descs, const uint64_t *__restrict__ knot_prefix,
-                        uint32_t nsys, uint64_t total_knots, int tri_layout, const SysDesc one) {
-    __shared__ CT sX[kPrecWarps][kPrecMaxN * (kPrecMaxN + 1)];
-    __shared__ __align__(16) CT sR[kPrecWarps][2][kPrecMaxN];
+                        uint32_t nsys, uint64_t total_knots, uint32_t per, int tri_layout, uint32_t classes,
+                        const SysDesc one) {
+    __shared__ CT sX[kPrecWarps][kPrecX];
+    __shared__ __align__(16) CT sR[kPrecWarps][kGjElems];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t gk = (uint64_t)blockIdx.x * kPrecWarps + warp;
+    uint64_t gk = ((uint64_t)blockIdx.x * kPrecWarps + warp) * per;
     if (gk >= total_knots) return;  // warp-uniform; no CTA-wide barrier below
+    const uint64_t end = min(gk + per, total_knots);
     // system owning global knot gk: last s with knot_prefix[s] <= gk (or the
     // one system passed by value)
-    uint32_t lo = 0, hi = nsys;
-    if (descs) {
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) / 2;
-            if (knot_prefix[mid] <= gk) lo = mid; else hi = mid;
+    uint32_t lo = descs ? find_system(knot_prefix, nsys, gk, lane) : 0u;
+    CT *s = sR[warp], *X = sX[warp];
+    while (gk < end) {
+        const uint32_t n = descs ? descs[lo].n : one.n, N = descs ? descs[lo].N : one.N;
+        const void *dS = descs ? descs[lo].S : one.S, *dP = descs ? descs[lo].P : one.P;
+        const uint32_t k = (uint32_t)(descs ? gk - knot_prefix[lo] : gk);
+        const uint32_t left = (uint32_t)min(end - gk, (uint64_t)(N - k));  // knots of this system in the range
+        uint32_t cnt = left;
+        if (np_class(n) >= 0 && ((classes >> np_class(n)) & 1u)) {  // a class of this launch
+            cnt = min(left, n <= 8 ? 4u : (n <= 16 ? 2u : 1u));
+            const TI *Sk = static_cast<const TI *>(dS) + (size_t)k * 3 * n * n + (size_t)n * n;
+            TO *row = static_cast<TO *>(const_cast<void *>(dP)) + (size_t)k * (tri_layout ? 3 : 1) * n * n;
+            if (n <= 8) invert_knots<TI, TO, CT, 8>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            else if (n <= 12) invert_knots<TI, TO, CT, 12>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            else if (n <= 16) invert_knots<TI, TO, CT, 16>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            else if (n <= 24) invert_knots<TI, TO, CT, 24>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            else invert_knots<TI, TO, CT, 32>(Sk, row, n, cnt, tri_layout, s, X, lane);
+        }
+        if (cnt == left) ++lo;  // the next knots are the next system's
+        gk += cnt;
+    }
+}
+
+// ---- FP32 batches: four rows a lane (gj_inverse_quad)
+
+constexpr int kQuadWarps = 2;
+// batches from this many knots on take it
+constexpr uint64_t kQuadFrom = 8192;
+// words of a warp's scratch: three rows of every block, and their transposes
+template <int NP>
+__host__ __device__ constexpr int quad_words() { return 3 * GjQuad<NP>::SCRATCH + GjQuad<NP>::BLOCKS * (NP * (NP + 1) + 1); }
+
+// Inverts `cnt` blocks of one system at once (cnt <= GjQuad::BLOCKS).  vw: rows of
+// an access (4 or 2 where n is a multiple and the addresses allow, else 1).
+template <int NP>
+__device__ __forceinline__ void invert_quads(const float *Sk, float *row, uint32_t n, uint32_t cnt, int tri_layout, uint32_t vw,
+                                             float *s, uint32_t lane) {
+    using G = GjQuad<NP>;
+    constexpr int P = NP / 2, LD = NP + 1, KX = NP * LD + 1;
+    const uint32_t g0 = lane / G::LANES, g = g0 < (uint32_t)G::BLOCKS ? g0 : 0u;
+    const uint32_t r = g0 < (uint32_t)G::BLOCKS ? lane % G::LANES : (uint32_t)G::LANES;
+    const uint32_t i0 = 4 * r, nn = n * n;
+    const bool mine = r < (uint32_t)G::LANES && g < cnt;
+    Sk += (size_t)g * 3 * nn + i0;
+    row += (size_t)g * (tri_layout ? 3 : 1) * nn + (tri_layout ? nn : 0) + i0;
+    bool in[4];  // rows of the block
+#pragma unroll
+    for (int t = 0; t < 4; ++t) in[t] = mine && i0 + t < n;
+    auto load4 = [&](const float *p, float (&v)[4], uint32_t c) {  // rows i0.. of column c; identity outside
+#pragma unroll
+        for (int t = 0; t < 4; ++t) v[t] = (c == i0 + t) ? 1.f : 0.f;
+        if (c >= n) return;
+        if (vw == 4) {
+            if (in[0]) {
+                const float4 x = __ldg(reinterpret_cast<const float4 *>(p));
+                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+            }
+        } else if (vw == 2) {
+#pragma unroll
+            for (int t = 0; t < 4; t += 2)
+                if (in[t]) {
+                    const float2 x = __ldg(reinterpret_cast<const float2 *>(p + t));
+                    v[t] = x.x; v[t + 1] = x.y;
+                }
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (in[t]) v[t] = __ldg(p + t);
+        }
+    };
+    unsigned long long A[4][P];
+    float diag[4], scale[4];
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+        float x[4], y[4];
+        load4(Sk + (size_t)(2 * p) * n, x, 2 * p);
+        load4(Sk + (size_t)(2 * p + 1) * n, y, 2 * p + 1);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) A[t][p] = pack2(x[t], y[t]);
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t) diag[t] = in[t] ? __ldg(Sk + (size_t)(i0 + t) * n + t) : 1.f;
+    float *buf = s + g * G::KS;
+    gj_inverse_quad<NP>(A, diag, scale, buf, r);
+    // symmetrise: X[c][row] of every block, and back transposed
+    float *X = s + 3 * G::SCRATCH + g * KX;
+    const float *D = buf + 2 * G::SCRATCH;
+    if (r < (uint32_t)G::LANES) {
+#pragma unroll
+        for (int p = 0; p < P; ++p)
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                X[(2 * p) * LD + i0 + t] = lo2(A[t][p]);
+                X[(2 * p + 1) * LD + i0 + t] = hi2(A[t][p]);
+            }
+    }
+    __syncwarp();
+    if (mine && i0 < n) {
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+            if ((uint32_t)c >= n) continue;
+            const float dc = D[c];
+            float v[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                v[t] = (((c & 1) ? hi2(A[t][c / 2]) : lo2(A[t][c / 2])) + X[(i0 + t) * LD + c]) * (0.5f * scale[t] * dc);
+            float *o = row + (size_t)c * n;
+            if (vw == 4) {
+                *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+            } else if (vw == 2) {
+                *reinterpret_cast<float2 *>(o) = make_float2(v[0], v[1]);
+                if (in[2]) *reinterpret_cast<float2 *>(o + 2) = make_float2(v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (in[t]) o[t] = v[t];
+            }
+            if (tri_layout) {
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    if (in[t]) {
+                        o[(int64_t)t - (int64_t)nn] = 0.f;
+                        o[t + nn] = 0.f;
+                    }
+            }
         }
     }
-    const SysDesc d = descs ? descs[lo] : one;
-    const uint32_t n = d.n, k = (uint32_t)(descs ? gk - knot_prefix[lo] : gk);
-    if (n == 0 || n > (uint32_t)kPrecMaxN) return;
-    const TI *Sk = static_cast<const TI *>(d.S) + (size_t)k * 3 * n * n + (size_t)n * n;
-    TO *row = static_cast<TO *>(const_cast<void *>(d.P)) + (size_t)k * (tri_layout ? 3 : 1) * n * n;
-    CT *s_raw = sR[warp][0], *s_t = sR[warp][1], *X = sX[warp];
-    if (n <= 8) invert_knot<TI, TO, CT, 8>(Sk, row, n, tri_layout, s_raw, s_t, X, lane);
-    else if (n <= 12) invert_knot<TI, TO, CT, 12>(Sk, row, n, tri_layout, s_raw, s_t, X, lane);
-    else if (n <= 16) invert_knot<TI, TO, CT, 16>(Sk, row, n, tri_layout, s_raw, s_t, X, lane);
-    else if (n <= 24) invert_knot<TI, TO, CT, 24>(Sk, row, n, tri_layout, s_raw, s_t, X, lane);
-    else invert_knot<TI, TO, CT, 32>(Sk, row, n, tri_layout, s_raw, s_t, X, lane);
+    __syncwarp();
+}
+
+// One launch per block-size class, so that an SM runs one class's code and a
+// narrow block does not pay for the registers of a wide one (all classes in one
+// kernel: 312 us where these take 190, 2048 systems of n in {6, 12, 14, 24}).
+// sys, knot_prefix: the class's systems and the knots before each; null: `one`.
+template <int NP>
+__global__ void __launch_bounds__(kQuadWarps * 32, NP <= 8 ? 12 : (NP <= 12 ? 9 : (NP <= 16 ? 8 : (NP <= 24 ? 6 : 4))))
+    block_jacobi_quad_kernel(const SysDesc *__restrict__ descs, const uint32_t *__restrict__ sys,
+                             const uint64_t *__restrict__ knot_prefix, uint32_t nsys, uint64_t total_knots, uint32_t per,
+                             int tri_layout, const SysDesc one) {
+    __shared__ __align__(16) float scratch[kQuadWarps][(quad_words<NP>() + 3) / 4 * 4];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t gk = ((uint64_t)blockIdx.x * kQuadWarps + warp) * per;
+    if (gk >= total_knots) return;  // warp-uniform; no CTA-wide barrier below
+    const uint64_t end = min(gk + per, total_knots);
+    uint32_t lo = sys ? find_system(knot_prefix, nsys, gk, lane) : 0u;
+    while (gk < end) {
+        const SysDesc *d = sys ? descs + sys[lo] : nullptr;
+        const uint32_t n = d ? d->n : one.n, N = d ? d->N : one.N;
+        const float *S = static_cast<const float *>(d ? d->S : one.S);
+        float *P = static_cast<float *>(const_cast<void *>(d ? d->P : one.P));
+        const uint32_t k = (uint32_t)(sys ? gk - knot_prefix[lo] : gk);
+        const uint32_t left = (uint32_t)min(end - gk, (uint64_t)(N - k));  // knots of this system in the range
+        const uint32_t cnt = min(left, (uint32_t)GjQuad<NP>::BLOCKS);
+        const uintptr_t at = reinterpret_cast<uintptr_t>(S) | reinterpret_cast<uintptr_t>(P);
+        const uint32_t vw = (n % 4 == 0 && (at & 15u) == 0) ? 4u : ((n % 2 == 0 && (at & 7u) == 0) ? 2u : 1u);
+        invert_quads<NP>(S + (size_t)k * 3 * n * n + (size_t)n * n, P + (size_t)k * (tri_layout ? 3 : 1) * n * n, n, cnt,
+                         tri_layout, vw, scratch[warp], lane);
+        if (cnt == left) ++lo;  // the next knots are the next system's
+        gk += cnt;
+    }
 }
 
 // kind: 0 float S -> float Phi^-1 (float arithmetic); 1 double -> double;
 // 2 double S -> float Phi^-1 (double arithmetic, for the refinement's inner solve)
 // d_descs == nullptr: the single system *one (total_knots = its N), passed to
 // the kernel by value (no descriptor upload).
+// cls: the batch by block-size class (null for a single system).
+int jacobi_class(uint32_t n) { return np_class(n); }
+
 cudaError_t launch_block_jacobi(int kind, const SysDesc *d_descs, const uint64_t *d_prefix,
                                 uint32_t nsys, uint64_t total_knots, int tri_layout,
-                                cudaStream_t stream, const SysDesc *one) {
+                                cudaStream_t stream, const SysDesc *one, const JacobiClasses *cls) {
     if (total_knots == 0) return cudaSuccess;
     SysDesc o;
     if (one) o = *one;
     else memset(&o, 0, sizeof(o));
-    const dim3 grid((unsigned)((total_knots + kPrecWarps - 1) / kPrecWarps)), block(kPrecWarps * 32);
+    uint32_t classes = 0x1f;  // left to the kernel with one row a lane
+    uint64_t rest = total_knots;
+    if (kind == 0) {
+        auto quad = [&](auto np) {
+            constexpr int NP = decltype(np)::value, c = np_class(NP);
+            const uint64_t knots = one ? (np_class(o.n) == c ? total_knots : 0) : cls->knots[c];
+            if (knots < kQuadFrom) return;
+            const uint32_t *sys = one ? nullptr : cls->sys + cls->first[c];
+            const uint64_t *prefix = one ? nullptr : cls->prefix + cls->first[c];
+            const uint32_t per = GjQuad<NP>::BLOCKS * (knots >= (uint64_t)GjQuad<NP>::BLOCKS * 4096 ? 2 : 1);
+            const uint64_t warps = (knots + per - 1) / per;
+            block_jacobi_quad_kernel<NP><<<(unsigned)((warps + kQuadWarps - 1) / kQuadWarps), kQuadWarps * 32, 0, stream>>>(
+                d_descs, sys, prefix, one ? 1u : cls->count[c], knots, per, tri_layout, o);
+            classes &= ~(1u << c);
+            rest -= knots;
+        };
+        quad(std::integral_constant<int, 24>());
+        quad(std::integral_constant<int, 32>());
+        quad(std::integral_constant<int, 16>());
+        quad(std::integral_constant<int, 12>());
+        quad(std::integral_constant<int, 8>());
+        if (rest == 0) return cudaGetLastError();
+    }
+    // knots a warp: side by side while the GPU has warps to spare, then several, as
+    // many as a warp inverts at once for a single system
+    const uint32_t most = d_descs ? 4u : (o.n <= 8 ? 4u : (o.n <= 16 ? 2u : 1u));
+    const uint32_t per = rest < 8192 ? 1u : (rest < 32768 ? (most < 2 ? most : 2u) : most);
+    const uint64_t warps = (total_knots + per - 1) / per;
+    const dim3 grid((unsigned)((warps + kPrecWarps - 1) / kPrecWarps)), block(kPrecWarps * 32);
     if (kind == 1)
         block_jacobi_kernel<double, double, double><<<grid, block, 0, stream>>>(
-            d_descs, d_prefix, nsys, total_knots, tri_layout, o);
+            d_descs, d_prefix, nsys, total_knots, per, tri_layout, classes, o);
     else if (kind == 2)
         block_jacobi_kernel<double, float, double><<<grid, block, 0, stream>>>(
-            d_descs, d_prefix, nsys, total_knots, tri_layout, o);
+            d_descs, d_prefix, nsys, total_knots, per, tri_layout, classes, o);
     else
         block_jacobi_kernel<float, float, float><<<grid, block, 0, stream>>>(
-            d_descs, d_prefix, nsys, total_knots, tri_layout, o);
+            d_descs, d_prefix, nsys, total_knots, per, tri_layout, classes, o);
     return cudaGetLastError();
 }
 
