@@ -240,14 +240,24 @@ std::vector<Pref> storage_prefs(bool f64, bool ptri, uint32_t storage) {
                 : std::vector<Pref>{{1, 2}, {0, 1}, {1, 1}, {2, 1}, {3, 2}, {3, 1}, {5, 2}, {5, 1}};
 }
 
+// Whether a kernel with rpt rows a thread holds blocks of size n: even n always;
+// odd n with an empty last row in the standard and recurrence forms on chip (the
+// single-reduction, refinement and streamed kernels have no such row).  Two rows
+// a thread share every vector load and fit tensor memory: 600 systems of n in {4,
+// 7, 13, 14, 21}, 10 to 100 knots, 666 us with one row a thread for the odd ones,
+// 377 so.
+bool rows_pair(uint32_t n, int st, int rpt, int alg) {
+    return n % (uint32_t)rpt == 0 || ((alg == 0 || alg == 3) && !streamed(st));
+}
+
 // A tuned shape for one system, if its variant exists and holds the system.
 bool tuned_shape(Registry *reg, bool f64, int acc, int np, bool ptri, uint32_t n, uint32_t N,
                  const TuneChoice &tc, Shape *out, bool fa = false) {
-    if (tc.rpt < 1 || n % tc.rpt || tc.C < 1 || tc.C > 16 || tc.threads == 0 || tc.threads % 32) return false;
+    if (tc.rpt < 1 || !rows_pair(n, tc.st, tc.rpt, tc.alg) || tc.C < 1 || tc.C > 16 || tc.threads == 0 || tc.threads % 32) return false;
     VariantInfo *vi = find_variant(reg, f64, acc, np, ptri, tc.st, tc.rpt, tc.alg, fa);
     if (!vi) return false;
     const uint32_t K = (N + tc.C - 1) / tc.C;
-    const uint32_t thr = (K * n + tc.rpt - 1) / tc.rpt;
+    const uint32_t thr = K * ((n + tc.rpt - 1) / tc.rpt);
     if ((!streamed(tc.st) && thr > tc.threads) || tc.threads > (uint32_t)vi->max_threads) return false;
     if (vi->v.smem_bytes(K, tc.C, tc.threads / 32) > (size_t)reg->max_smem_optin) return false;
     out->vi = vi;
@@ -373,7 +383,7 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
         prefs.insert(prefs.begin(), Pref{4, 2});
     // the first cluster size from `from` up at which storage pf holds the system
     auto fit = [&](const Pref &pf, uint32_t from, Shape *o) -> bool {
-        if (pf.rpt > 1 && (n % pf.rpt) != 0) return false;
+        if (!rows_pair(n, pf.st, pf.rpt, alg)) return false;
         VariantInfo *vi = find_variant(reg, f64 && !refine, acc, np, ptri, pf.st, pf.rpt, alg, fa);
         if (!vi) return false;
         uint32_t cap = cfg.max_threads ? cfg.max_threads : (uint32_t)vi->max_threads;
@@ -383,7 +393,7 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
         for (uint32_t C = c_lo; C <= c_hi; ++C) {
             if (C > 8 && (C & (C - 1))) continue;  // large clusters: powers of two only
             const uint32_t K = (N + C - 1) / C;
-            const uint32_t thr = (K * n + pf.rpt - 1) / pf.rpt;
+            const uint32_t thr = K * ((n + pf.rpt - 1) / pf.rpt);
             if (thr > cap && !streamed(pf.st)) continue;
             // CTA sizes are rounded to 64 threads so that systems of similar
             // size share a launch (streamed rows: up to the cap, in row groups)
@@ -403,7 +413,7 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
     };
     for (uint32_t from : {first_lo, 1u}) {
         for (const Pref &pf : prefs) {
-            if (pf.rpt > 1 && (n % pf.rpt) != 0) continue;
+            if (!rows_pair(n, pf.st, pf.rpt, alg)) continue;
             if (streamed(pf.st) && lone && ptri && cfg.storage == GBDPCG_STORAGE_AUTO &&
                 cfg.algorithm == GBDPCG_ALGO_AUTO && cfg.cluster_size == 0 && plain_fits(reg, f64, n, N)) {
                 s.plain = true;
@@ -1862,7 +1872,7 @@ std::vector<Candidate> tune_candidates(gbdpcg_plan_s *p, const PlanClass &base,
         if (v.fa != (int)p->fused) continue;  // pairs run on the variants built for them
         if (want_st >= 0 && v.st != want_st) continue;
         bool rows_ok = true;
-        for (uint32_t i : items) rows_ok &= p->descs[i].n % v.rpt == 0;
+        for (uint32_t i : items) rows_ok &= rows_pair(p->descs[i].n, v.st, v.rpt, v.alg);
         if (!rows_ok) continue;
         uint32_t cap = std::min<uint32_t>((uint32_t)vi.max_threads,
                                           p->cfg.max_threads ? p->cfg.max_threads : 1024u);
@@ -1875,7 +1885,7 @@ std::vector<Candidate> tune_candidates(gbdpcg_plan_s *p, const PlanClass &base,
                 const uint32_t K = (N + C - 1) / C;
                 ok &= N > (C - 1) * K;  // every CTA of the cluster owns a knot
                 kmax = std::max(kmax, K);
-                thr = std::max(thr, (K * n + v.rpt - 1) / v.rpt);
+                thr = std::max(thr, K * ((n + v.rpt - 1) / v.rpt));
             }
             uint32_t threads = (thr + 31) / 32 * 32;
             if (streamed(v.st)) threads = std::min(threads, cap / 32 * 32);  // row groups beyond the cap

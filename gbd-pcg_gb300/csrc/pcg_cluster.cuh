@@ -7,8 +7,10 @@
 //     system from a device work queue (an atomic counter over a host-sorted,
 //     longest-first list).  C comes from the launch's cluster dimension.
 //   * CTA `rank` owns the contiguous knots [kb, ke), kb = rank*K, K = ceil(N/C).
-//   * Thread t of a CTA owns RPT consecutive matrix rows (RPT = 2 only for even
-//     n, so both rows lie in one knot and share every vector load).  The rows
+//   * Thread t of a CTA owns RPT consecutive matrix rows of one knot, which share
+//     every vector load.  With RPT = 2 and odd n a knot takes n + 1 rows: the last
+//     thread's second row is empty (its matrix, vectors and products are zero, and
+//     it is neither read nor written in global memory).  The rows
 //     of S (3 blocks) and of Phi^-1 (1 or 3 blocks) are held for the whole
 //     solve on chip; ST selects where: 0 both in registers, 1 S in registers
 //     and Phi^-1 in shared memory, 2 both in shared memory, 3 hybrid (two S
@@ -450,27 +452,28 @@ __device__ __forceinline__ void stage_elem(TO *dst, const TI *src) {
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Stage the block rows of knots [kb, kb+nk) (blk = NB n^2 elements each,
-// column-major n x NB n) into the column-interleaved layout M[c*R + k*n + i].
+// column-major n x NB n) into the column-interleaved layout M[c*R + k*ne + i]
+// (ne: rows a knot takes there, n or n + 1).
 template <typename TO, typename TI>
 __device__ __forceinline__ void stage_rows(TO *M, uint32_t R, const TI *__restrict__ g, uint32_t nk,
-                                           uint32_t n, uint32_t blk, uint32_t tid, uint32_t nthr) {
+                                           uint32_t n, uint32_t ne, uint32_t blk, uint32_t tid, uint32_t nthr) {
     for (uint32_t e = tid; e < nk * blk; e += nthr) {
         const uint32_t kl = e / blk, w = e - kl * blk;
         const uint32_t c = w / n, i = w - c * n;
-        stage_elem(M + (size_t)c * R + kl * n + i, g + e);
+        stage_elem(M + (size_t)c * R + kl * ne + i, g + e);
     }
 }
 
 // Stage block `blk_off` (n^2 elements) of each of the block rows of knots
-// [kb, kb+nk) (stride elements apart) into M[c*R + k*n + i].
+// [kb, kb+nk) (stride elements apart) into M[c*R + k*ne + i].
 template <typename TO, typename TI>
 __device__ __forceinline__ void stage_block(TO *M, uint32_t R, const TI *__restrict__ g, uint32_t nk,
-                                            uint32_t n, uint32_t stride, uint32_t tid, uint32_t nthr) {
+                                            uint32_t n, uint32_t ne, uint32_t stride, uint32_t tid, uint32_t nthr) {
     const uint32_t blk = n * n;
     for (uint32_t e = tid; e < nk * blk; e += nthr) {
         const uint32_t kl = e / blk, w = e - kl * blk;
         const uint32_t c = w / n, i = w - c * n;
-        stage_elem(M + (size_t)c * R + kl * n + i, g + (size_t)kl * stride + w);
+        stage_elem(M + (size_t)c * R + kl * ne + i, g + (size_t)kl * stride + w);
     }
 }
 
@@ -1147,8 +1150,9 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
         const SysDesc d = lp.descs ? lp.descs[lp.order ? lp.order[item] : item] : lp.one;
         const uint32_t n = d.n, N = d.N;
         const uint32_t K = (N + C - 1) / C;
-        if (n == 0 || N == 0 || n > (uint32_t)NP || K > lp.kmax || (size_t)K * n > (size_t)nthr * RPT ||
-            (RPT > 1 && (n % RPT) != 0) || (!FA && (d.flags & SYS_FWD_ADJ))) {
+        const uint32_t ne = RPT == 2 ? (n + 1) & ~1u : n;  // rows a knot takes
+        if (n == 0 || N == 0 || n > (uint32_t)NP || K > lp.kmax || (size_t)K * ne > (size_t)nthr * RPT ||
+            (!FA && (d.flags & SYS_FWD_ADJ))) {
             if (rank == 0 && tid == 0) {
                 SysResult res = {};
                 res.status = -1;
@@ -1161,8 +1165,9 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
         }
         const uint32_t kb = min(rank * K, N), ke = min(kb + K, N), nk = ke - kb;
         const uint32_t row0 = tid * RPT;
-        const uint32_t lk = row0 / n, i = row0 - lk * n;  // rows i .. i+RPT-1 of local knot lk
+        const uint32_t lk = row0 / ne, i = row0 - lk * ne;  // rows i .. i+RPT-1 of local knot lk
         const bool act = lk < nk;
+        const bool act1 = act && (RPT == 1 || i + 1 < n);  // its last row too
         const uint32_t k = kb + lk;
         const bool relres = (d.flags & SYS_EXIT_RELRES) != 0;
         const T *__restrict__ S = static_cast<const T *>(d.S);
@@ -1171,11 +1176,11 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
         const T *__restrict__ lam0 =
             (d.flags & SYS_LAMBDA0_ZERO) ? nullptr : static_cast<const T *>(d.lambda0);
         const uint32_t blkS = 3 * n * n, blkP = NBP * n * n;
-        const uint32_t R = (K * n + 1) & ~1u;  // row stride of staged matrices (even)
+        const uint32_t R = (K * ne + 1) & ~1u;  // row stride of staged matrices (even)
         const bool has_left = nk > 0 && kb > 0, has_right = nk > 0 && ke < N;
         const bool first_knot = act && lk == 0 && kb > 0, last_knot = act && lk + 1 == nk && ke < N;
-        // halo bytes the neighbours send to this CTA before a reduction (n values each)
-        const uint32_t halo_in = ((has_left ? n : 0u) + (has_right ? n : 0u)) * (uint32_t)sizeof(T);
+        // halo bytes the neighbours send to this CTA before a reduction (a knot's rows each)
+        const uint32_t halo_in = ((has_left ? ne : 0u) + (has_right ? ne : 0u)) * (uint32_t)sizeof(T);
         // this CTA's block rows of S and Phi^-1 into L2 at once: the staging
         // loads below then wait on L2, not on HBM, round after round
         if (tid == 0 && nk > 0 && !adj_pass()) {
@@ -1199,19 +1204,19 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                 for (int j = 0; j < NP; ++j)
 #pragma unroll
                     for (int q = 0; q < RPT; ++q)
-                        Sr[q][b * NP + j] = (present && (uint32_t)j < n)
+                        Sr[q][b * NP + j] = (present && (q == 0 || act1) && (uint32_t)j < n)
                                                 ? __ldg(Sk + (b * n + j) * n + i + q)
                                                 : T(0);
             }
             if constexpr (S_HYB)
-                if (!adj_pass()) stage_block(ms, R, S + (size_t)kb * blkS + 2 * n * n, nk, n, blkS, tid, nthr);
+                if (!adj_pass()) stage_block(ms, R, S + (size_t)kb * blkS + 2 * n * n, nk, n, ne, blkS, tid, nthr);
         } else if constexpr (S_TM) {
             const T *Sk = S + (size_t)k * blkS;
 #pragma unroll
             for (int j = 0; j < NP; ++j)
 #pragma unroll
                 for (int q = 0; q < RPT; ++q)
-                    Sr[q][j] = (act && (uint32_t)j < n) ? __ldg(Sk + (n + j) * n + i + q) : T(0);
+                    Sr[q][j] = ((q == 0 ? act : act1) && (uint32_t)j < n) ? __ldg(Sk + (n + j) * n + i + q) : T(0);
             __syncwarp();  // tcgen05 stores are warp-wide
             // The off-diagonal S blocks and Phi^-1 go to TMEM in 8-column pieces
             // ("rounds": 2 blocks x RPT rows x NPT/8 pieces of S, then RPT x NPT/8
@@ -1227,7 +1232,7 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                     const bool is_s = r < RS;
                     const int rr = is_s ? r % (RPT * NC) : r - RS;
                     const int bi = is_s ? r / (RPT * NC) : 0, q = rr / NC, cc = rr % NC;
-                    const bool present = is_s ? (bi == 0 ? pres0 : pres2) : act;
+                    const bool present = (is_s ? (bi == 0 ? pres0 : pres2) : act) && (q == 0 || act1);
                     const T *src = is_s ? Sk + (size_t)(2 * bi) * n * n + i + q : Pk + i + q;
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
@@ -1253,7 +1258,7 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
             tmem_wait_st();
         } else {
             const T *Sg = S + (size_t)kb * blkS;
-            if (!adj_pass()) stage_rows(ms, R, Sg, nk, n, blkS, tid, nthr);
+            if (!adj_pass()) stage_rows(ms, R, Sg, nk, n, ne, blkS, tid, nthr);
         }
         if constexpr (S_TM) {
             // Phi^-1 went to tensor memory with the off-diagonal S blocks
@@ -1267,20 +1272,20 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                 for (int j = 0; j < NP; ++j)
 #pragma unroll
                     for (int q = 0; q < RPT; ++q)
-                        Pr[q][b * NP + j] = (present && (uint32_t)j < n)
+                        Pr[q][b * NP + j] = (present && (q == 0 || act1) && (uint32_t)j < n)
                                                 ? __ldg(Pk + (b * n + j) * n + i + q)
                                                 : T(0);
             }
         } else {
             const T *Pg = P + (size_t)kb * blkP;
-            if (!adj_pass()) stage_rows(mp, R, Pg, nk, n, blkP, tid, nthr);
+            if (!adj_pass()) stage_rows(mp, R, Pg, nk, n, ne, blkP, tid, nthr);
         }
         const int sb0 = (k == 0) ? 1 : 0, sb1 = (k + 1 == N) ? 2 : 3;
         auto matS = [&](const T *x, T(&y)[RPT]) {
             if constexpr (S_REG) reg_matvec<T, NP, 3, RPT>(Sr, x, y);
             else if constexpr (S_TM) tmem_matvec<NP>(Sr, trow, x, y);
-            else if constexpr (S_HYB) hyb_matvec<T, NP, RPT>(Sr, ms, R, lk * n + i, sb1 == 3, x, n, y);
-            else smem_matvec<T, NP, 3, RPT>(ms, R, lk * n + i, sb0, sb1, x, n, y);
+            else if constexpr (S_HYB) hyb_matvec<T, NP, RPT>(Sr, ms, R, lk * ne + i, sb1 == 3, x, n, y);
+            else smem_matvec<T, NP, 3, RPT>(ms, R, lk * ne + i, sb0, sb1, x, n, y);
         };
         auto matP = [&](const T *x, T(&y)[RPT]) {
             if constexpr (S_TM) {
@@ -1289,12 +1294,13 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                 if constexpr (PTRI) reg_matvec<T, NP, 3, RPT>(Pr, x, y);
                 else reg_matvec<T, NP, 1, RPT>(Pr, x + NP, y);
             } else {
-                if constexpr (PTRI) smem_matvec<T, NP, 3, RPT>(mp, R, lk * n + i, sb0, sb1, x, n, y);
-                else smem_matvec<T, NP, 1, RPT>(mp, R, lk * n + i, 0, 1, x + NP, n, y);
+                if constexpr (PTRI) smem_matvec<T, NP, 3, RPT>(mp, R, lk * ne + i, sb0, sb1, x, n, y);
+                else smem_matvec<T, NP, 1, RPT>(mp, R, lk * ne + i, 0, 1, x + NP, n, y);
             }
         };
-        // y = S p over this thread's rows (zero for a thread without rows); with
-        // tensor memory every thread of a warp takes part in the loads
+        // y = S p over this thread's rows (zero for a thread without rows and for an
+        // empty last row, which in shared memory holds what the staging found there);
+        // with tensor memory every thread of a warp takes part in the loads
         auto matS_rows = [&](T(&y)[RPT]) {
             if constexpr (S_TM) {
                 matS(vp + (act ? lk : 0u) * NP, y);
@@ -1308,6 +1314,8 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
 #pragma unroll
                     for (int q = 0; q < RPT; ++q) y[q] = T(0);
                 }
+                if constexpr (RPT == 2 && !S_REG)
+                    if (!act1) y[RPT - 1] = T(0);
             }
         };
         // z = Phi^-1 r over this thread's rows, the same way
@@ -1324,6 +1332,8 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
 #pragma unroll
                     for (int q = 0; q < RPT; ++q) z[q] = T(0);
                 }
+                if constexpr (RPT == 2 && !P_REG)
+                    if (!act1) z[RPT - 1] = T(0);
             }
         };
         T *my_p = vp + (lk + 1) * NP + i;  // this thread's rows in the windows
@@ -1341,10 +1351,11 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
 #pragma unroll
         for (int q = 0; q < RPT; ++q) {
             const size_t row = (size_t)k * n + i + q;
-            gam[q] = act ? (adj0 ? static_cast<const T *>(d.lambda)[row] - static_cast<const T *>(d.lstar)[row]
-                                 : gamma[row])
-                         : T(0);
-            lam[q] = (act && lam_init) ? lam_init[row] : T(0);
+            const bool have = q == 0 ? act : act1;
+            gam[q] = have ? (adj0 ? static_cast<const T *>(d.lambda)[row] - static_cast<const T *>(d.lstar)[row]
+                                  : gamma[row])
+                          : T(0);
+            lam[q] = (have && lam_init) ? lam_init[row] : T(0);
             if (act) my_p[q] = lam[q];
         }
         if (lam_init) {
@@ -1624,10 +1635,9 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
         if constexpr (FA) dd = reload_outputs(lp, item);
         else dd = OutFields{d.lambda, d.mu, d.dS, d.lam_fwd, d.flags, d.result, d.result_adj};
         T *lam_out = static_cast<T *>(adj ? dd.mu : dd.lambda);
-        if (act) {
 #pragma unroll
-            for (int q = 0; q < RPT; ++q) lam_out[(size_t)k * n + i + q] = lam[q];
-        }
+        for (int q = 0; q < RPT; ++q)
+            if (q == 0 ? act : act1) lam_out[(size_t)k * n + i + q] = lam[q];
         if (rank == 0 && tid == 0) {
             if (C > 1)  // a reduction wait of some CTA of the cluster gave up
                 for (uint32_t c = 0; c < C; ++c)
@@ -1652,7 +1662,7 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
             T lfi[RPT];
 #pragma unroll
             for (int q = 0; q < RPT; ++q) {
-                lfi[q] = act ? lf[(size_t)k * n + i + q] : T(0);
+                lfi[q] = (q == 0 ? act : act1) ? lf[(size_t)k * n + i + q] : T(0);
                 if (act) {
                     my_r[q] = lam[q];  // mu
                     my_p[q] = lfi[q];
@@ -1682,7 +1692,7 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
 #pragma unroll
                         for (int q = 0; q < RPT; ++q) {
                             const T g = present ? T(-0.5) * fma_rn(lam[q], lw[j], lfi[q] * mw[j]) : T(0);
-                            dS[(size_t)k * blkS + (b * n + j) * n + i + q] = g;
+                            if (q == 0 || act1) dS[(size_t)k * blkS + (b * n + j) * n + i + q] = g;
                         }
                     }
                 }
@@ -1855,7 +1865,7 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, false, ST, RPT>::max_thre
             }
         } else {
             const T *Sg = S + (size_t)kb * blkS;
-            stage_rows(ms, R, Sg, nk, n, blkS, tid, nthr);
+            stage_rows(ms, R, Sg, nk, n, n, blkS, tid, nthr);
         }
         if constexpr (P_REG) {
             const T *Pk = P + (size_t)k * blkP;
@@ -1866,7 +1876,7 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, false, ST, RPT>::max_thre
                     Pr[q][j] = (act && (uint32_t)j < n) ? __ldg(Pk + j * n + i + q) : T(0);
         } else {
             const T *Pg = P + (size_t)kb * blkP;
-            stage_rows(mp, R, Pg, nk, n, blkP, tid, nthr);
+            stage_rows(mp, R, Pg, nk, n, n, blkP, tid, nthr);
         }
         const int sb0 = (k == 0) ? 1 : 0, sb1 = (k + 1 == N) ? 2 : 3;
         auto matS = [&](const T *x, T(&y)[RPT]) {

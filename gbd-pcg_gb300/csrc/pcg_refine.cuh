@@ -221,7 +221,7 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
             tmem_wait_st();
         } else {
             const double *Sg = S64 + (size_t)kb * blkS;
-            stage_rows(ms, R, Sg, nk, n, blkS, tid, nthr);
+            stage_rows(ms, R, Sg, nk, n, n, blkS, tid, nthr);
         }
         if constexpr (S_TM) {
             // Phi^-1 went to tensor memory with the off-diagonal S blocks
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__((RegBudget<float, double, NP, false, ST, RPT>:
                     Pr[q][j] = (act && (uint32_t)j < n) ? __ldg(Pk + j * n + i + q) : T(0);
         } else {
             const T *Pg = P + (size_t)kb * blkP;
-            stage_rows(mp, R, Pg, nk, n, blkP, tid, nthr);
+            stage_rows(mp, R, Pg, nk, n, n, blkP, tid, nthr);
         }
         // S x and Phi^-1 x over this thread's rows (zero for a thread without rows);
         // with tensor memory every thread of a warp takes part in the loads

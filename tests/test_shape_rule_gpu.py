@@ -35,7 +35,8 @@ def _solve(gb, O, handle, n, N, count, storage):
 @pytest.mark.parametrize("n,N,count,want", [
     (14, 36, 400, TMEM), (14, 27, 400, SPLIT), (14, 27, 152, TMEM), (14, 27, 153, SPLIT), (14, 60, 100, TMEM),
     (24, 64, 76, TMEM), (24, 64, 300, TMEM), (24, 10, 300, SPLIT), (8, 64, 300, SPLIT), (8, 96, 300, TMEM),
-    (6, 128, 300, TMEM), (6, 85, 300, SPLIT), (2, 3, 1, TMEM)])
+    (6, 128, 300, TMEM), (6, 85, 300, SPLIT), (2, 3, 1, TMEM), (13, 36, 400, TMEM), (13, 27, 400, SPLIT),
+    (23, 64, 300, TMEM), (7, 96, 300, TMEM), (7, 40, 400, SPLIT), (1, 5, 1, TMEM)])
 def test_rule(gb, oracle_mod, handle, n, N, count, want):
     l, lam, err = _solve(gb, oracle_mod, handle, n, N, count, gb.STORAGE_AUTO)
     assert l["storage"] == want, l
@@ -45,10 +46,10 @@ def test_rule(gb, oracle_mod, handle, n, N, count, want):
     assert err <= 1.5 * err_s + 1e-6
 
 
-def test_no_tensor_memory_for_odd_n_fp64_or_cbtd(gb, oracle_mod, handle):
+def test_no_tensor_memory_for_fp64_or_cbtd(gb, oracle_mod, handle):
     import torch
     O = oracle_mod
-    for n, dt, layout in ((13, np.float32, "compact"), (14, np.float64, "compact"), (14, np.float32, "cbtd")):
+    for n, dt, layout in ((14, np.float64, "compact"), (14, np.float32, "cbtd"), (13, np.float64, "compact")):
         sy = O.generate(n, 36, 3)
         t = [torch.from_numpy(a.astype(dt)).cuda() for a in (sy.cbtd(dt), O.block_jacobi(sy.D, layout), sy.gamma)]
         lam = torch.zeros_like(t[2])
