@@ -26,8 +26,8 @@
 // in shared memory and forms its Gram product as a register tile per lane;
 // S_kk is symmetrised through shared memory (0.5 (S + S^T), exactly
 // symmetric), and the formation can invert S_kk in the same warp (the
-// block-Jacobi Phi^-1).  The back-substitution's lane i reads column i of
-// A_k and B_k.
+// block-Jacobi Phi^-1).  In the back-substitution lane l reads column l of
+// [A_k | B_k].
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -48,28 +48,6 @@ constexpr int kKktMaxN = 32;  // n, m <= 32
 // memory either way in the formation)
 template <typename T>
 constexpr int kkt_warps() { return sizeof(T) == 8 ? 2 : 4; }
-
-// elements of one 16-byte vector
-template <typename T>
-__host__ __device__ constexpr int kkt_vw() { return 16 / (int)sizeof(T); }
-
-// 16-byte global loads of consecutive elements (the back-substitution's columns)
-template <typename T>
-struct Vec16;
-template <>
-struct Vec16<float> {
-    __device__ static void get(const float *p, float (&v)[4]) {
-        const float4 t = *reinterpret_cast<const float4 *>(p);
-        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-    }
-};
-template <>
-struct Vec16<double> {
-    __device__ static void get(const double *p, double (&v)[2]) {
-        const double2 t = *reinterpret_cast<const double2 *>(p);
-        v[0] = t.x; v[1] = t.y;
-    }
-};
 
 // Shared-memory layout of one warp for the formation: Mt[l][r] = M[r][l] with
 // M = [A_k | B_k] (n x (n + m)), i.e. row l of Mt is column l of A_k (l < n)
@@ -339,54 +317,69 @@ __global__ void __launch_bounds__(W * 32, sizeof(T) == 4 ? (NP <= 24 ? 7 : 5) : 
     }
 }
 
-// s + sum_j col[j] w[j], j ascending.  A lane reads its own contiguous column:
-// 16-byte loads when both pointers are 16-byte aligned and n is a multiple of
-// the vector width (a quarter of the L1 requests of scalar loads; the
-// products are added in the same order either way).
-template <typename T>
+// s + sum_j col[j] w[j], j ascending, VW elements an access (n a multiple of VW,
+// both addresses aligned to it).
+template <typename T, int VW>
 __device__ __forceinline__ T col_dot(const T *col, const T *w, uint32_t n, T s) {
-    constexpr int VW = kkt_vw<T>();
-    if ((n % VW) == 0 && ((reinterpret_cast<uintptr_t>(col) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
-        for (uint32_t j = 0; j < n; j += VW) {
-            T a[VW], b[VW];
-            Vec16<T>::get(col + j, a);
-            Vec16<T>::get(w + j, b);
+    for (uint32_t j = 0; j < n; j += VW) {
+        T a[VW], b[VW];
+        load_vec<T, VW>(col + j, a);
+        load_vec<T, VW>(w + j, b);
 #pragma unroll
-            for (int u = 0; u < VW; ++u) s += a[u] * b[u];
-        }
-        return s;
+        for (int u = 0; u < VW; ++u) s += a[u] * b[u];
     }
-    for (uint32_t j = 0; j < n; ++j) s += col[j] * w[j];
     return s;
 }
 
-template <typename T, int kKktWarps = kkt_warps<T>()>
+// Back-substitution: a lane per column of [A_k | B_k] (element l of x_k for l < n,
+// of u_k beyond), GL lanes a knot, so that both blocks go in one pass and a warp
+// takes two knots of n + m <= 16 or four of n + m <= 8.  From 25 columns on (TWO)
+// the columns of A_k go first, then those of B_k: together their lines outgrow the
+// L1 of an SM's 64 warps (n=24 m=12: 55 us against 50; n=24 m=8 46 / 44, n=16 m=8
+// 31.3 / 32.0).  A lane reads its own
+// contiguous column with accesses of 16 or 8 bytes where n and the addresses allow.
+//
+// What bounds it: HBM and, for short columns, the L1 requests (a column is 24 to
+// 128 bytes).  Measured, us, before (one pass for A_k, one for B_k, one element an
+// access unless n is a multiple of 4) and now: n=14 m=7 N=40001 22.9 -> 19.7, n=6
+// m=3 N=60000 21.1 -> 10.4, n=13 m=6 N=60000 30.7 -> 25.3, n=22 m=11 N=60000 56.3 ->
+// 42.4; n=24 m=12 N=65536 (50.4) and FP64, bound by its pipe, are as they were.
+template <typename T, int GL, int VW, bool TWO, int kKktWarps>
 __global__ void __launch_bounds__(kKktWarps * 32)
     kkt_backsub_kernel(const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ Qd,
                        const T *__restrict__ Rd, const T *__restrict__ q, const T *__restrict__ r,
                        const T *__restrict__ lambda, uint32_t n, uint32_t m, uint32_t N, T *__restrict__ x,
                        T *__restrict__ u) {
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t k = blockIdx.x * kKktWarps + warp;  // knots 0..N (x) and 0..N-1 (u)
-    if (k > N) return;
-    if (lane < n) {
-        const uint32_t i = lane;
-        T s = q[(size_t)k * n + i];
-        if (k < N) {  // + (A_k^T lambda_k)_i = sum_j A_k[j][i] lambda_k[j]; column i of A_k is contiguous
-            const T *Acol = A + (size_t)k * n * n + (size_t)i * n;
-            const T *lk = lambda + (size_t)k * n;
-            s = col_dot(Acol, lk, n, s);
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t k = (blockIdx.x * kKktWarps + (threadIdx.x >> 5)) * (32 / GL) + lane / GL;
+    if (k > N) return;  // knots 0..N (x) and 0..N-1 (u)
+    const T *lk = lambda + (size_t)k * n;
+    if constexpr (TWO) {
+        const uint32_t l = lane;
+        if (l < n) {
+            T s = q[(size_t)k * n + l];
+            if (k < N) s = col_dot<T, VW>(A + ((size_t)k * n + l) * n, lk, n, s);
+            if (k > 0) s -= lambda[(size_t)(k - 1) * n + l];
+            x[(size_t)k * n + l] = -s / Qd[(size_t)k * n + l];
         }
-        if (k > 0) s -= lambda[(size_t)(k - 1) * n + i];
-        x[(size_t)k * n + i] = -s / Qd[(size_t)k * n + i];
-    }
-    if (k < N && lane < m) {
-        const uint32_t i = lane;
-        T s = r[(size_t)k * m + i];
-        const T *Bcol = B + (size_t)k * n * m + (size_t)i * n;
-        const T *lk = lambda + (size_t)k * n;
-        s = col_dot(Bcol, lk, n, s);
-        u[(size_t)k * m + i] = -s / Rd[(size_t)k * m + i];
+        if (k < N && l < m) {
+            const T s = col_dot<T, VW>(B + ((size_t)k * m + l) * n, lk, n, r[(size_t)k * m + l]);
+            u[(size_t)k * m + l] = -s / Rd[(size_t)k * m + l];
+        }
+        return;
+    } else for (uint32_t l = lane % GL; l < (k < N ? n + m : n); l += GL) {
+        const bool is_x = l < n;
+        const size_t e = is_x ? (size_t)k * n + l : (size_t)k * m + (l - n);
+        T s = is_x ? q[e] : r[e];
+        const T d = is_x ? Qd[e] : Rd[e];
+        if (k < N)  // + (A_k^T lambda_k)_i = sum_j A_k[j][i] lambda_k[j], B_k^T lambda_k alike
+            s = col_dot<T, VW>(is_x ? A + ((size_t)k * n + l) * n : B + ((size_t)k * m + (l - n)) * n, lk, n, s);
+        if (is_x) {
+            if (k > 0) s -= lambda[(size_t)(k - 1) * n + l];
+            x[e] = -s / d;
+        } else {
+            u[e] = -s / d;
+        }
     }
 }
 
@@ -466,9 +459,26 @@ int kkt_backsub(const T *A, const T *B, const T *Qd, const T *Rd, const T *q, co
     const void *p[] = {A, B, Qd, Rd, q, r, lambda, x, u};
     int rc = check(p, 9, n, m, N);
     if (rc) return rc;
-    constexpr int W = kkt_warps<T>();
-    kkt_backsub_kernel<T><<<(N + 1 + W - 1) / W, W * 32, 0, st>>>(A, B, Qd, Rd, q, r,
-                                                                                           lambda, n, m, N, x, u);
+    constexpr int W = 4;
+    const uintptr_t at =
+        reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(lambda);
+    constexpr uint32_t V16 = 16 / sizeof(T);
+    auto go = [&](auto gl, auto two, auto vw) {
+        constexpr int GL = decltype(gl)::value, VW = decltype(vw)::value, K = W * (32 / GL);
+        kkt_backsub_kernel<T, GL, VW, decltype(two)::value, W>
+            <<<N / K + 1, W * 32, 0, st>>>(A, B, Qd, Rd, q, r, lambda, n, m, N, x, u);
+    };
+    auto width = [&](auto gl, auto two) {
+        if (n % V16 == 0 && (at & 15u) == 0) return go(gl, two, std::integral_constant<int, (int)V16>());
+        if constexpr (sizeof(T) == 4)
+            if (n % 2 == 0 && (at & 7u) == 0) return go(gl, two, std::integral_constant<int, 2>());
+        go(gl, two, std::integral_constant<int, 1>());
+    };
+    const std::false_type one;
+    if (n + m <= 8) width(std::integral_constant<int, 8>(), one);
+    else if (n + m <= 16) width(std::integral_constant<int, 16>(), one);
+    else if (n + m <= 24) width(std::integral_constant<int, 32>(), one);
+    else width(std::integral_constant<int, 32>(), std::true_type());
     return launched("kkt_backsub");
 }
 

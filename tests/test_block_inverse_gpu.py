@@ -107,3 +107,38 @@ def test_formation_alignments(gb, oracle_mod, n, m, N):
         got.append([o.clone() for o in outs])
     for o in got[1:]:
         assert all(torch.equal(a, b) for a, b in zip(got[0], o))
+
+
+@pytest.mark.parametrize("f64", [False, True])
+@pytest.mark.parametrize("n,m,N", [(1, 1, 1), (5, 3, 9), (6, 3, 130), (8, 8, 3), (12, 12, 21), (13, 6, 2), (14, 7, 65), (16, 9, 5),
+                                   (22, 11, 7), (24, 1, 4), (32, 32, 3)])
+def test_back_substitution_alignments(gb, oracle_mod, n, m, N, f64):
+    """x and u are the same bits from arrays of every alignment, and within the rounding of
+    a sum of n + 2 terms and a division, (n + 4) u relative to the terms, of the 64-bit result."""
+    import torch
+    dt = torch.float64 if f64 else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(n * 100 + m)
+    rnd = lambda k: torch.randn(k, device="cuda", generator=g, dtype=dt)  # noqa: E731
+    pos = lambda k: 0.5 + torch.rand(k, device="cuda", generator=g, dtype=dt)  # noqa: E731
+    src = [rnd(n * n * N), rnd(n * m * N), pos(n * (N + 1)), pos(m * N), rnd(n * (N + 1)), rnd(m * N), rnd(n * N)]
+    got = []
+    for shift in (0, 2, 1):
+        ins = [torch.empty(t.numel() + 4, device="cuda", dtype=dt)[shift:shift + t.numel()].copy_(t) for t in src]
+        x, u = (torch.full((k,), float("nan"), device="cuda", dtype=dt) for k in (n * (N + 1), m * N))
+        gb.kkt_backsub(*ins, n, m, N, x, u)
+        got.append((x, u))
+    assert all(torch.equal(a, b) for o in got[1:] for a, b in zip(got[0], o))
+    A, B, Q, R, q, r, lam = (t.double() for t in src)
+    A, B, L = A.reshape(N, n, n), B.reshape(N, m, n), lam.reshape(N, n)  # [knot, column, row]
+    xs, ax = q.reshape(N + 1, n).clone(), q.reshape(N + 1, n).abs()
+    xs[:N] += (A @ L[:, :, None])[:, :, 0]
+    ax[:N] += (A.abs() @ L.abs()[:, :, None])[:, :, 0]
+    xs[1:] -= L
+    ax[1:] += L.abs()
+    us = r.reshape(N, m) + (B @ L[:, :, None])[:, :, 0]
+    au = r.reshape(N, m).abs() + (B.abs() @ L.abs()[:, :, None])[:, :, 0]
+    eps = 2.0 ** -53 if f64 else 2.0 ** -24
+    for v, w, a, d in ((got[0][0], xs, ax, Q), (got[0][1], us, au, R)):
+        w, a = -w.reshape(-1) / d, a.reshape(-1) / d
+        # (the 64-bit reference rounds as often as an FP64 result)
+        assert bool(((v.double() - w).abs() <= (2 if f64 else 1) * (n + 4) * eps * a).all())
