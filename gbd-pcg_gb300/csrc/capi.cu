@@ -466,6 +466,9 @@ struct gbdpcg_handle_s {
     DevBuf ws;          // fixed-size: result slots, one descriptor (never reallocated)
     DevBuf host_io;     // host-pointer solve: S, Pinv, gamma, lambda
     DevBuf plain_scratch;  // plain algorithm: r, p, dot partials
+    // result of the handle's single solves: pinned host memory that the kernels
+    // write, so that reading it after the stream has ended takes no copy
+    SysResult *result = nullptr;
     SysResult *d_last = nullptr;
     cudaStream_t last_stream = nullptr;
     bool last_f64 = false;
@@ -478,6 +481,7 @@ struct gbdpcg_handle_s {
     cudaMemPool_t pool = nullptr;
     ~gbdpcg_handle_s() {
         if (pool) cudaMemPoolDestroy(pool);
+        if (result) cudaFreeHost(result);
     }
 };
 
@@ -711,7 +715,7 @@ int solve_grid(gbdpcg_handle_s *h, bool f64, const SysDesc &d, uint32_t layout, 
 // One system, device pointers; result left in h->d_last.
 int solve_one(gbdpcg_handle_s *h, bool f64, const SysDesc &d0, const gbdpcg_config &cfg,
               uint32_t layout, cudaStream_t stream, bool refine = false) {
-    SysResult *d_res = h->ws.as<SysResult>();
+    SysResult *d_res = h->result;
     int rc;
     SysDesc d = d0;
     d.result = 0;
@@ -1002,6 +1006,11 @@ int gbdpcg_create(gbdpcg_handle_t *handle, int device) {
     if (rc) return rc;
     rc = h->ws.ensure(kWorkspaceBytes);
     if (rc) return rc;
+    if (cudaHostAlloc(reinterpret_cast<void **>(&h->result), sizeof(SysResult), cudaHostAllocMapped | cudaHostAllocPortable) !=
+        cudaSuccess) {
+        h->result = nullptr;
+        return fail(GBDPCG_ERR_NO_MEMORY, "cudaHostAlloc of the result");
+    }
     *handle = h.release();
     return GBDPCG_SUCCESS;
 }
@@ -1048,10 +1057,8 @@ int gbdpcg_solve_dev_f64(gbdpcg_handle_t h, const double *d_S, const double *d_P
 int gbdpcg_last_result(gbdpcg_handle_t h, gbdpcg_result *result) {
     if (!h || !result || !h->d_last) return fail(GBDPCG_ERR_INVALID_ARGUMENT, "no result");
     HandleScope scope(h->device);
-    SysResult r;
-    GB_CUDA(cudaMemcpyAsync(&r, h->d_last, sizeof(r), cudaMemcpyDeviceToHost, h->last_stream));
     GB_CUDA(cudaStreamSynchronize(h->last_stream));
-    to_public(r, result);
+    to_public(*h->d_last, result);
     return GBDPCG_SUCCESS;
 }
 
