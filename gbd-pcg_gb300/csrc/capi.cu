@@ -276,17 +276,20 @@ int acc_kind(bool f64_system, bool refine, uint32_t dot_precision) {
     return (int)dot_precision;
 }
 
-// Cluster size a lone system (latency, not throughput) starts its search at:
-// C = 1 up to 40 knots (no cluster barriers), else about 16 knots a CTA (8 for
-// FP64 rows), rounded up to a power of two.  Measured on n = 14: N = 32 is
-// fastest at C = 1, N = 128 at C = 8 (FP32) and C = 16 (FP64).
-uint32_t lone_cluster_pref(bool f64_rows, uint32_t N) {
-    if (N <= 40) return 1;
-    const uint32_t per = f64_rows ? 8 : 16;
-    const uint32_t want = (N + per - 1) / per;
+// Cluster size a lone system (latency, not throughput) starts its search at,
+// rounded up to a power of two.  FP32: C = 1 up to 40 knots (no cluster
+// barriers), else about 16 knots a CTA; measured on n = 14: N = 32 is fastest at
+// C = 1, N = 128 at C = 8.  FP64 rows, bound by each SM's FP64 pipe: about 128
+// rows a CTA.  Measured, us, C = 1 / 2 / 4 / 8 / 16: n=6 N=20 89 / 105 / 107 / 111
+// / 113; n=14 N=16 195 / 150 / 160 / 162 / 168; n=14 N=32 - / 228 / 170 / 178 /
+// 183; n=20 N=30 1018 / 543 / 263 / 240 / 250; n=24 N=60 C = 8 318, 16 271; n=14
+// N=128 C = 8 265, 16 199.
+uint32_t lone_cluster_pref(bool f64_rows, uint32_t n, uint32_t N) {
+    if (!f64_rows && N <= 40) return 1;
+    const uint64_t want = f64_rows ? ((uint64_t)n * N + 127) / 128 : (N + 15) / 16;
     uint32_t p = 1;
-    while (p < want) p <<= 1;
-    return std::min<uint32_t>(16, p);
+    while (p < want && p < 16) p <<= 1;
+    return p;
 }
 
 // Whether the plain algorithm's N CTAs of 64 threads can all be resident at
@@ -721,7 +724,7 @@ int solve_one(gbdpcg_handle_s *h, bool f64, const SysDesc &d0, const gbdpcg_conf
     d.result = 0;
     Shape sh;
     rc = choose_shape(h->reg, f64, d.n, d.N, layout, cfg, &sh, refine, nullptr,
-                      lone_cluster_pref(f64 && !refine, d.N), true);
+                      lone_cluster_pref(f64 && !refine, d.n, d.N), true);
     if (rc) return rc;
     if (grid_pays(sh, d, cfg, refine)) {
         bool done = false;
@@ -1168,7 +1171,7 @@ static int solve_host(bool f64, const void *S, const void *P, const void *g, voi
     if (direct && mat >= ((size_t)1 << 20)) {
         Shape sh;
         SysDesc d = make_desc(S, P, g, l, l, n, N, c, build_layout, 0);
-        if (choose_shape(h->reg, f64, n, N, build_layout, c, &sh, false, nullptr, lone_cluster_pref(f64, N), true) ==
+        if (choose_shape(h->reg, f64, n, N, build_layout, c, &sh, false, nullptr, lone_cluster_pref(f64, n, N), true) ==
                 GBDPCG_SUCCESS &&
             np_for(n) && grid_pays(sh, d, c, false))
             direct = false;
