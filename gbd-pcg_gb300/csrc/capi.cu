@@ -10,7 +10,8 @@
 //     queue), the classes spread over a few streams, all captured in one CUDA
 //     graph that also resets the queues;
 //   * the single-system entry points (host and device pointers), which pass
-//     the system descriptor by value and need no queue;
+//     the system descriptor by value and need no queue, and the whole-GPU
+//     kernel for the long ones among them;
 //   * the plain algorithm (one CTA per knot, cooperative launch) for n > 32.
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -13,7 +13,7 @@ struct KernelVariant {
     int st;      // storage: 0 S and Phi^-1 in registers, 1 S in registers and Phi^-1 in
                  // shared memory, 2 both in shared memory, 3 hybrid, 4 tensor memory,
                  // 5 streamed from global memory
-    int rpt;     // matrix rows per thread (2 needs an even n)
+    int rpt;     // matrix rows per thread (2 and odd n: an empty row a knot; even n only for alg 1, 2 and st 5)
     int alg;     // 0 two reductions per iteration, 1 single reduction (block-diagonal Phi^-1),
                  // 2 FP32 inner PCG with FP64 refinement, 3 recurrence form (three barriers
                  // per iteration)

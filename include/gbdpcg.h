@@ -104,15 +104,17 @@ enum {
 };
 /* where the cluster solver keeps the matrix rows: AUTO picks; REGISTERS: S and
  * Phi^-1 rows in registers; SHARED: both staged in shared memory; SPLIT: S rows
- * in registers (two per thread for even n), Phi^-1 in shared memory; HYBRID:
+ * in registers (two per thread), Phi^-1 in shared memory; HYBRID:
  * the sub-diagonal and diagonal blocks of S in registers, its super-diagonal
  * block and Phi^-1 in shared memory (more rows per SM; FP32, block-diagonal
  * Phi^-1); TMEM: the diagonal block of S in registers, its off-diagonal
  * blocks in the SM's tensor memory, Phi^-1 in shared memory (the most rows
- * per SM; FP32, block-diagonal Phi^-1, even n; one CTA per SM); STREAM: no
+ * per SM; FP32, block-diagonal Phi^-1; one CTA per SM); STREAM: no
  * storage, the rows are read from global memory (L2 or HBM) in every
  * product, so a cluster holds any system whose vectors fit its shared memory
- * (three vectors of its knots; AUTO's last choice before the plain algorithm) */
+ * (three vectors of its knots; AUTO's last choice for batches; a lone system
+ * that only this storage or the plain algorithm would hold takes, with AUTO
+ * everywhere, a kernel over the whole GPU instead, except under stream capture) */
 enum {
     GBDPCG_STORAGE_AUTO = 0,
     GBDPCG_STORAGE_REGISTERS = 1,
