@@ -782,7 +782,7 @@ def block_jacobi_build(plan, descs, hbm_gbs, reps=5):
     nbytes = sum(2 * 4 * n * n * N for (n, N, _, _, _) in descs)
     return {"ms": ms, "knots": knots, "bytes": nbytes, "gbs": nbytes / (ms / 1e3) / 1e9,
             "frac_of_hbm": nbytes / (ms / 1e3) / 1e9 / hbm_gbs,
-            "note": "one warp per knot, rotating Gauss-Jordan in registers: issue-bound, not HBM-bound"}
+            "note": "4 to 16 knots a warp, Gauss-Jordan in registers: bound by instruction fetch and issue, not HBM"}
 
 
 def _gen_ill(n, N, seed):
