@@ -469,7 +469,11 @@ struct gbdpcg_handle_s {
     Registry *reg = nullptr;
     DevBuf ws;          // fixed-size: result slots, one descriptor (never reallocated)
     DevBuf host_io;     // host-pointer solve: S, Pinv, gamma, lambda
-    DevBuf plain_scratch;  // plain algorithm: r, p, dot partials
+    // plain algorithm: r, p, dot partials.  The grid's CTAs exchange them, so two
+    // solves at once in the same scratch would disagree on the exit and wait for
+    // one another for ever: each waits for the one before it, on whatever stream.
+    DevBuf plain_scratch;
+    cudaEvent_t plain_done = nullptr;
     // result of a single solve whose caller waits for it: pinned host memory that
     // the kernel writes, so that reading it after the stream has ended takes no
     // copy (49.3 -> 43.5 us for a call of n=14 N=32).  A solve that nobody waits for
@@ -487,6 +491,7 @@ struct gbdpcg_handle_s {
     std::mutex pool_mu;
     cudaMemPool_t pool = nullptr;
     ~gbdpcg_handle_s() {
+        if (plain_done) cudaEventDestroy(plain_done);
         if (pool) cudaMemPoolDestroy(pool);
         if (result) cudaFreeHost(result);
     }
@@ -743,7 +748,19 @@ int solve_one(gbdpcg_handle_s *h, bool f64, const SysDesc &d0, const gbdpcg_conf
     h->d_last = d_res;
     h->last_stream = stream;
     if (sh.plain) {
-        return launch_plain(h, f64, d, d_res, stream, h->plain_scratch);
+        // (a captured solve cannot wait for work outside its graph: its replays are
+        // ordered by whoever launches them)
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return launch_plain(h, f64, d, d_res, stream, h->plain_scratch);
+        }
+        if (!h->plain_done) GB_CUDA(cudaEventCreateWithFlags(&h->plain_done, cudaEventDisableTiming));
+        else GB_CUDA(cudaStreamWaitEvent(stream, h->plain_done, 0));
+        rc = launch_plain(h, f64, d, d_res, stream, h->plain_scratch);
+        if (rc) return rc;
+        GB_CUDA(cudaEventRecord(h->plain_done, stream));
+        return GBDPCG_SUCCESS;
     }
     LaunchParams lp;
     memset(&lp, 0, sizeof(lp));
