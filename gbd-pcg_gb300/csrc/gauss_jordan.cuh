@@ -1,4 +1,4 @@
-// Inverse of small symmetric positive definite blocks held one row per lane
+// Inverse of small symmetric blocks, positive definite in earnest, one row per lane
 // (shared by the block-Jacobi builder and the fused Schur formation):
 // Gauss-Jordan elimination without pivoting.
 //
@@ -9,12 +9,19 @@
 // (16-byte broadcast loads) from its own.  Registers are renamed by a shift of
 // two columns every two steps, so all indices are compile-time constants while
 // the loop stays rolled, and FP32 rows are updated two columns an instruction
-// (fma.rn.f32x2).  The pivot row needs no selects: with m = 1 - 1/a_kk in its
-// lane the common update is a_kj / a_kk.  For |a_kk| <= 1 that m is exact and the
-// one rounding of the update is the quotient's, so the rows are scaled by powers
-// of two (exactly) to a diagonal in [1/4, 1): every pivot of a positive definite
-// block is then at most 1, and the result is bit for bit that of the elimination
-// that divides the pivot row.  A zero pivot leaves its column unscaled.
+// (fma.rn.f32x2).
+//
+// The pivot row needs no selects: with m = 1 - 1/a_kk in its lane the common
+// update is a_kj / a_kk.  For pivots in [u, 2) (u = 2^-24 in FP32, 2^-53 in
+// FP64) that m is exact and the one rounding of the update is the quotient's.  So the
+// rows are scaled by powers of two (exactly) to a diagonal in [1/4, 1), and a
+// block whose first diagonal element is negative is inverted as its negative:
+// every pivot of a positive or negative definite block is then at most 1, and the
+// result is bit for bit that of the elimination that divides the pivot row.
+// Other blocks (indefinite, singular, nearly singular) leave that range at some
+// pivot; the elimination notes it, and the caller inverts the block again by
+// gj_invert_any, which divides the pivot row and neither scales nor negates: a zero
+// pivot then leaves its column unscaled.
 //
 // What bounds it is the issue of instructions: about 42 a column of an n = 24
 // block (12 f32x2 FMAs, 12 shared-memory accesses) where scaling the pivot row in
@@ -97,23 +104,46 @@ __device__ __forceinline__ double mul_pow2(double x, double s, double t) {
     return x * s * t;
 }
 
+// How far a pivot lies outside [u, 2): the largest over a block's pivots stays
+// within kPivotRange where all of them are inside (integer operations: NaN,
+// infinities, zero and negative pivots are outside too).
+__device__ __forceinline__ uint32_t pivot_off(float piv) { return __float_as_uint(piv) - 0x33800000u; }
+__device__ __forceinline__ uint32_t pivot_off(double piv) { return (uint32_t)__double2hiint(piv) - 0x3ca00000u; }
+template <typename CT>
+constexpr uint32_t kPivotRange = sizeof(CT) == 4 ? 0x40000000u - 0x33800000u - 1u : 0x40000000u - 0x3ca00000u - 1u;
+
+// Negative where d is (integer work: an FP64 comparison would wait for that pipe).
+__device__ __forceinline__ int sign_word(float d) { return __float_as_int(d); }
+__device__ __forceinline__ int sign_word(double d) { return __double2hiint(d); }
+
 // lanes a block of NP rows takes
 __host__ __device__ constexpr int gj_lanes(int NP) { return NP <= 8 ? 8 : (NP <= 16 ? 16 : 32); }
 // shared memory of a warp, in elements: three rows of 32
 constexpr int kGjElems = 96;
 
 // In: a = row r of the block (identity rows and columns beyond n; anything for
-// r >= NP), diag = its diagonal element.  Out: a = row r of (D A D)^-1 for the
-// power-of-two diagonal D, D_r (returned), and D in s[2 GL ..]: (A^-1)_rc =
-// a[c] D_r D_c.  s: this group's 3 GL elements (16-byte aligned) of the warp's
-// scratch; r: lane in the group.  Called by whole warps.
+// r >= NP), diag = its diagonal element, real = r < n.  Out: a = row r of
+// (D A D)^-1 for the power-of-two diagonal D, D_r (returned), and D in s[2 GL ..]:
+// (A^-1)_rc = a[c] D_r D_c; FP32, negative first diagonal element: a and the D_r
+// returned are both negated.  `ok`: every pivot of the block was in range.  s: this
+// group's 3 GL elements (16-byte aligned) of the warp's scratch; r: lane in the
+// group.  Called by whole warps.
 template <typename CT, int NP, int GL>
-__device__ __forceinline__ CT gj_inverse(CT (&a)[NP], CT diag, CT *s, uint32_t r) {
+__device__ __forceinline__ CT gj_inverse(CT (&a)[NP], CT diag, bool real, CT *s, uint32_t r, bool &ok) {
     static_assert(NP % 2 == 0 && NP <= GL, "pairs of columns; a lane per row");
     constexpr int W = PrecVec<CT>::W;
     const bool row = r < (uint32_t)NP;
-    const CT scale = row ? pow2_scale(diag) : CT(0);
+    uint32_t off = 0;
+    const bool negative = __shfl_sync(0xffffffffu, sign_word(diag), 0, GL) < 0;
+    CT scale = row ? pow2_scale(diag) : CT(0);
     if (row) s[2 * GL + r] = scale;
+    // FP32 negates by the scale; FP64, whose scaling is integer work, the elements
+    if constexpr (sizeof(CT) == 4) {
+        if (real && negative) scale = -scale;
+    } else if (real && negative) {
+#pragma unroll
+        for (int c = 0; c < NP; ++c) a[c] = -a[c];
+    }
     __syncwarp();
 #pragma unroll
     for (int c = 0; c < NP; c += W) {
@@ -148,7 +178,7 @@ __device__ __forceinline__ CT gj_inverse(CT (&a)[NP], CT diag, CT *s, uint32_t r
             bool pivot = r == k;
             pivot_row(pivot, s);
             float piv = lo2(T[0]);
-            if (piv == 0.f) piv = 1.f;
+            off = max(off, pivot_off(piv));
             float inv = 1.f / piv, m = pivot ? 1.f - inv : lo2(A[0]) * inv;
             unsigned long long nm = pack2(-m, -m);
 #pragma unroll
@@ -159,7 +189,7 @@ __device__ __forceinline__ CT gj_inverse(CT (&a)[NP], CT diag, CT *s, uint32_t r
             pivot = r == k + 1;
             pivot_row(pivot, s + GL);
             piv = hi2(T[0]);
-            if (piv == 0.f) piv = 1.f;
+            off = max(off, pivot_off(piv));
             inv = 1.f / piv;
             m = pivot ? 1.f - inv : hi2(A[0]) * inv;
             nm = pack2(-m, -m);
@@ -183,8 +213,8 @@ __device__ __forceinline__ CT gj_inverse(CT (&a)[NP], CT diag, CT *s, uint32_t r
                 for (int c = 0; c < NP; c += 2) *reinterpret_cast<double2 *>(buf + c) = make_double2(a[c], a[c + 1]);
             }
             __syncwarp();
-            CT piv = buf[0];
-            if (piv == CT(0)) piv = CT(1);
+            const CT piv = buf[0];
+            off = max(off, pivot_off(piv));
             const CT inv = CT(1) / piv;
             // pivot ? 1 - inv : a[0] inv, in one FP64 instruction (x + -0 = x)
             const CT m = fma(pivot ? CT(-1) : a[0], inv, pivot ? CT(1) : CT(-0.0));
@@ -198,9 +228,46 @@ __device__ __forceinline__ CT gj_inverse(CT (&a)[NP], CT diag, CT *s, uint32_t r
             }
             a[NP - 1] = pivot ? inv : -m;
         }
+        if (real && negative) {
+#pragma unroll
+            for (int c = 0; c < NP; ++c) a[c] = -a[c];
+        }
     }
     __syncwarp();
+    ok = off <= kPivotRange<CT>;
     return scale;
+}
+
+// Inverts the block in X (element (r, c) at X[c ld + r], n <= 32) of any kind, with
+// the pivot row divided; its inverse, symmetrised, to P (with zero blocks on both
+// sides of it for `sides`).  The rows stay in shared memory, lane r working on row r,
+// so that a kernel whose blocks seldom need it keeps its registers.  s: n elements.
+// Called by whole warps.
+template <typename CT, typename TO>
+__device__ __forceinline__ void gj_invert_any(CT *X, uint32_t ld, TO *P, bool sides, uint32_t n, CT *s, uint32_t r) {
+    const bool row = r < n;
+    const uint32_t nn = n * n;
+    for (uint32_t k = 0; k < n; ++k) {
+        __syncwarp();
+        CT piv = X[k * ld + k];
+        if (piv == CT(0)) piv = CT(1);
+        const CT inv = CT(1) / piv, m = row ? X[k * ld + r] : CT(0);
+        if (row) s[r] = r == k ? inv : X[r * ld + k] * inv;
+        __syncwarp();
+        for (uint32_t c = 0; row && c < n; ++c) {
+            CT *x = X + c * ld + r;
+            *x = r == k ? s[c] : (c == k ? -(m * inv) : *x - m * s[c]);
+        }
+    }
+    __syncwarp();
+    for (uint32_t c = 0; row && c < n; ++c) {
+        P[c * n + r] = TO(CT(0.5) * (X[c * ld + r] + X[r * ld + c]));
+        if (sides) {
+            (P - nn)[c * n + r] = TO(0);
+            (P + nn)[c * n + r] = TO(0);
+        }
+    }
+    __syncwarp();
 }
 
 // ---- four rows a lane (FP32)
@@ -220,20 +287,27 @@ struct GjQuad {
     static constexpr int SCRATCH = BLOCKS * KS;  // one row of every block
 };
 
-// In: A[t][p] = columns 2p, 2p + 1 of row 4r + t, diag its diagonal elements.
-// Out: A = rows of (D A D)^-1, scale[t] = D of its rows.  buf: this block's row
+// In: A[t][p] = columns 2p, 2p + 1 of row 4r + t, diag its diagonal elements,
+// real[t]: not an identity row, negative: the block's first diagonal element is.
+// Out: A = rows of (s D A D)^-1, scale[t] = s D of its rows, D and s as in
+// gj_inverse; returns whether every pivot was in range.  buf: this block's row
 // buffer, the second one GjQuad::SCRATCH words on and D's a further SCRATCH on;
 // r >= LANES: a lane without rows (its registers are arbitrary but finite, it
 // stores nothing and reads a valid buffer).
 template <int NP>
-__device__ __forceinline__ void gj_inverse_quad(unsigned long long (&A)[4][NP / 2], const float (&diag)[4], float (&scale)[4],
-                                                float *buf, uint32_t r) {
+__device__ __forceinline__ bool gj_inverse_quad(unsigned long long (&A)[4][NP / 2], const float (&diag)[4],
+                                                const bool (&real)[4], bool negative, float (&scale)[4], float *buf,
+                                                uint32_t r) {
     using G = GjQuad<NP>;
     constexpr int P = NP / 2;
     const bool live = r < (uint32_t)G::LANES;
 #pragma unroll
     for (int t = 0; t < 4; ++t) scale[t] = pow2_scale(diag[t]);
     if (live) *reinterpret_cast<float4 *>(buf + 2 * G::SCRATCH + 4 * r) = make_float4(scale[0], scale[1], scale[2], scale[3]);
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+        if (real[t] && negative) scale[t] = -scale[t];
+    uint32_t off = 0;
     __syncwarp();
 #pragma unroll
     for (int p = 0; p < P; p += 2) {
@@ -258,8 +332,8 @@ __device__ __forceinline__ void gj_inverse_quad(unsigned long long (&A)[4][NP / 
             }
             __syncwarp();
             const unsigned long long t0 = *reinterpret_cast<const unsigned long long *>(row);
-            float piv = (q & 1) ? hi2(t0) : lo2(t0);
-            if (piv == 0.f) piv = 1.f;
+            const float piv = (q & 1) ? hi2(t0) : lo2(t0);
+            off = max(off, pivot_off(piv));
             const float inv = 1.f / piv;
             unsigned long long nm[4], end[4];
             float last[4];
@@ -294,6 +368,7 @@ __device__ __forceinline__ void gj_inverse_quad(unsigned long long (&A)[4][NP / 
         }
     }
     __syncwarp();
+    return off <= kPivotRange<float>;
 }
 
 }  // namespace gbdpcg

@@ -300,7 +300,13 @@ __global__ void __launch_bounds__(W * 32, sizeof(T) == 4 ? (NP <= 24 ? 7 : 5) : 
             a[cc] = (mine && (uint32_t)cc < n) ? Yg[cc * ldt + rr] : ((uint32_t)cc == rr ? T(1) : T(0));
         const T diag = mine ? Yg[rr * ldt + rr] : T(1);
         T *sg = s + g * 3 * GL;
-        const T h = T(0.5) * gbdpcg::gj_inverse<T, NP, GL>(a, diag, sg, rr);  // ends with a warp sync: Y is free
+        bool ok;
+        const T h = T(0.5) * gbdpcg::gj_inverse<T, NP, GL>(a, diag, mine, sg, rr, ok);  // ends with a warp sync: Y is free
+        if (!__all_sync(0xffffffffu, ok)) {
+            for (uint32_t k = k0; k < kend; ++k)
+                gbdpcg::gj_invert_any(Y + (k - k0) * NP * ldt, ldt, Pinv + (size_t)k * nn, false, n, s, lane);
+            return;
+        }
         const T *D = sg + 2 * GL;
         T *Xg = Y + g * NP * ldt;
         if (rr < (uint32_t)NP) {

@@ -67,9 +67,9 @@ __device__ __forceinline__ uint32_t find_system(const uint64_t *__restrict__ kno
 
 // Inverts `cnt` blocks of one system at once (cnt <= 32 / GL): block g's S_kk at
 // Sk + g strideS, its row of Phi^-1 at row + g strideP.  Groups from cnt on run on
-// the identity and write nothing.
+// the identity and write nothing.  Whether this lane's block is inverted (gj_inverse).
 template <typename TI, typename TO, typename CT, int NP>
-__device__ __forceinline__ void invert_knots(const TI *Sk, TO *row, uint32_t n, uint32_t cnt, int tri_layout, CT *s, CT *X,
+__device__ __forceinline__ bool invert_knots(const TI *Sk, TO *row, uint32_t n, uint32_t cnt, int tri_layout, CT *s, CT *X,
                                              uint32_t lane) {
     constexpr int GL = gj_lanes(NP), LD = GL + 1;
     const uint32_t g = lane / GL, r = lane % GL;
@@ -85,7 +85,8 @@ __device__ __forceinline__ void invert_knots(const TI *Sk, TO *row, uint32_t n, 
     const CT diag = mine ? CT(Sk[(size_t)r * n + r]) : CT(1);
     s += g * 3 * GL;
     X += g * GL * LD;
-    const CT h = CT(0.5) * gj_inverse<CT, NP, GL>(a, diag, s, r);  // (lanes without a row: 0, not used)
+    bool ok;
+    const CT h = CT(0.5) * gj_inverse<CT, NP, GL>(a, diag, mine, s, r, ok);  // (lanes without a row: 0, not used)
     const CT *D = s + 2 * GL;
     // symmetrise through a shared-memory transpose: X[r][c] = a[c] of lane r
     if (r < (uint32_t)NP) {
@@ -108,13 +109,35 @@ __device__ __forceinline__ void invert_knots(const TI *Sk, TO *row, uint32_t n, 
         }
     }
     __syncwarp();
+    return ok;
+}
+
+// Inverts knots [gk, end) of the batch again, one after another (gj_invert_any): for
+// a warp that met a block that is not definite.  sys: the systems in the order of
+// knot_prefix (null: 0, 1, ..); descs null: `one`.  s: 32 elements, X: 32 x 32.
+template <typename TI, typename TO, typename CT>
+__device__ __noinline__ void invert_range_any(const SysDesc *descs, const uint32_t *sys, const uint64_t *knot_prefix,
+                                              uint32_t nsys, uint64_t gk, uint64_t end, int tri_layout, const SysDesc *one,
+                                              CT *s, CT *X) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = descs ? find_system(knot_prefix, nsys, gk, lane) : 0u;
+    for (; gk < end; ++gk) {
+        while (descs && lo + 1 < nsys && knot_prefix[lo + 1] <= gk) ++lo;
+        const SysDesc *d = descs ? descs + (sys ? sys[lo] : lo) : one;
+        const uint32_t n = d->n, nn = n * n, k = (uint32_t)(descs ? gk - knot_prefix[lo] : gk);
+        if (np_class(n) < 0) continue;
+        const TI *Sk = static_cast<const TI *>(d->S) + (size_t)k * 3 * nn + nn;
+        TO *row = static_cast<TO *>(const_cast<void *>(d->P)) + (size_t)k * (tri_layout ? 3 : 1) * nn + (tri_layout ? nn : 0);
+        for (uint32_t e = lane; e < nn; e += 32) X[e] = CT(Sk[e]);
+        gj_invert_any<CT, TO>(X, n, row, tri_layout, n, s, lane);
+    }
 }
 
 template <typename TI, typename TO, typename CT>
 __global__ void __launch_bounds__(kPrecWarps * 32, sizeof(CT) == 4 ? 5 : 4)
     block_jacobi_kernel(const SysDesc *__restrict__ descs, const uint64_t *__restrict__ knot_prefix,
                         uint32_t nsys, uint64_t total_knots, uint32_t per, int tri_layout, uint32_t classes,
-                        const SysDesc one) {
+                        const __grid_constant__ SysDesc one) {
     __shared__ CT sX[kPrecWarps][kPrecX];
     __shared__ __align__(16) CT sR[kPrecWarps][kGjElems];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -125,6 +148,7 @@ __global__ void __launch_bounds__(kPrecWarps * 32, sizeof(CT) == 4 ? 5 : 4)
     // one system passed by value)
     uint32_t lo = descs ? find_system(knot_prefix, nsys, gk, lane) : 0u;
     CT *s = sR[warp], *X = sX[warp];
+    bool ok = true;
     while (gk < end) {
         const uint32_t n = descs ? descs[lo].n : one.n, N = descs ? descs[lo].N : one.N;
         const void *dS = descs ? descs[lo].S : one.S, *dP = descs ? descs[lo].P : one.P;
@@ -135,14 +159,18 @@ __global__ void __launch_bounds__(kPrecWarps * 32, sizeof(CT) == 4 ? 5 : 4)
             cnt = min(left, n <= 8 ? 4u : (n <= 16 ? 2u : 1u));
             const TI *Sk = static_cast<const TI *>(dS) + (size_t)k * 3 * n * n + (size_t)n * n;
             TO *row = static_cast<TO *>(const_cast<void *>(dP)) + (size_t)k * (tri_layout ? 3 : 1) * n * n;
-            if (n <= 8) invert_knots<TI, TO, CT, 8>(Sk, row, n, cnt, tri_layout, s, X, lane);
-            else if (n <= 12) invert_knots<TI, TO, CT, 12>(Sk, row, n, cnt, tri_layout, s, X, lane);
-            else if (n <= 16) invert_knots<TI, TO, CT, 16>(Sk, row, n, cnt, tri_layout, s, X, lane);
-            else if (n <= 24) invert_knots<TI, TO, CT, 24>(Sk, row, n, cnt, tri_layout, s, X, lane);
-            else invert_knots<TI, TO, CT, 32>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            if (n <= 8) ok &= invert_knots<TI, TO, CT, 8>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            else if (n <= 12) ok &= invert_knots<TI, TO, CT, 12>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            else if (n <= 16) ok &= invert_knots<TI, TO, CT, 16>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            else if (n <= 24) ok &= invert_knots<TI, TO, CT, 24>(Sk, row, n, cnt, tri_layout, s, X, lane);
+            else ok &= invert_knots<TI, TO, CT, 32>(Sk, row, n, cnt, tri_layout, s, X, lane);
         }
         if (cnt == left) ++lo;  // the next knots are the next system's
         gk += cnt;
+    }
+    if (!__all_sync(0xffffffffu, ok)) {
+        gk = ((uint64_t)blockIdx.x * kPrecWarps + warp) * per;
+        invert_range_any<TI, TO, CT>(descs, nullptr, knot_prefix, nsys, gk, min(gk + per, total_knots), tri_layout, &one, s, X);
     }
 }
 
@@ -155,10 +183,11 @@ constexpr uint64_t kQuadFrom = 8192;
 template <int NP>
 __host__ __device__ constexpr int quad_words() { return 3 * GjQuad<NP>::SCRATCH + GjQuad<NP>::BLOCKS * (NP * (NP + 1) + 1); }
 
-// Inverts `cnt` blocks of one system at once (cnt <= GjQuad::BLOCKS).  vw: rows of
+// Inverts `cnt` blocks of one system at once (cnt <= GjQuad::BLOCKS); whether this
+// lane's block is inverted.  vw: rows of
 // an access (4 or 2 where n is a multiple and the addresses allow, else 1).
 template <int NP>
-__device__ __forceinline__ void invert_quads(const float *Sk, float *row, uint32_t n, uint32_t cnt, int tri_layout, uint32_t vw,
+__device__ __forceinline__ bool invert_quads(const float *Sk, float *row, uint32_t n, uint32_t cnt, int tri_layout, uint32_t vw,
                                              float *s, uint32_t lane) {
     using G = GjQuad<NP>;
     constexpr int P = NP / 2, LD = NP + 1, KX = NP * LD + 1;
@@ -206,7 +235,8 @@ __device__ __forceinline__ void invert_quads(const float *Sk, float *row, uint32
 #pragma unroll
     for (int t = 0; t < 4; ++t) diag[t] = in[t] ? __ldg(Sk + (size_t)(i0 + t) * n + t) : 1.f;
     float *buf = s + g * G::KS;
-    gj_inverse_quad<NP>(A, diag, scale, buf, r);
+    const bool negative = __shfl_sync(0xffffffffu, diag[0], g * G::LANES) < 0.f;
+    const bool ok = gj_inverse_quad<NP>(A, diag, in, negative, scale, buf, r);
     // symmetrise: X[c][row] of every block, and back transposed
     float *X = s + 3 * G::SCRATCH + g * KX;
     const float *D = buf + 2 * G::SCRATCH;
@@ -251,6 +281,7 @@ __device__ __forceinline__ void invert_quads(const float *Sk, float *row, uint32
         }
     }
     __syncwarp();
+    return ok;
 }
 
 // One launch per block-size class, so that an SM runs one class's code and a
@@ -261,13 +292,14 @@ template <int NP>
 __global__ void __launch_bounds__(kQuadWarps * 32, NP <= 8 ? 12 : (NP <= 12 ? 9 : (NP <= 16 ? 8 : (NP <= 24 ? 6 : 4))))
     block_jacobi_quad_kernel(const SysDesc *__restrict__ descs, const uint32_t *__restrict__ sys,
                              const uint64_t *__restrict__ knot_prefix, uint32_t nsys, uint64_t total_knots, uint32_t per,
-                             int tri_layout, const SysDesc one) {
+                             int tri_layout, const __grid_constant__ SysDesc one) {
     __shared__ __align__(16) float scratch[kQuadWarps][(quad_words<NP>() + 3) / 4 * 4];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint64_t gk = ((uint64_t)blockIdx.x * kQuadWarps + warp) * per;
     if (gk >= total_knots) return;  // warp-uniform; no CTA-wide barrier below
     const uint64_t end = min(gk + per, total_knots);
     uint32_t lo = sys ? find_system(knot_prefix, nsys, gk, lane) : 0u;
+    bool ok = true;
     while (gk < end) {
         const SysDesc *d = sys ? descs + sys[lo] : nullptr;
         const uint32_t n = d ? d->n : one.n, N = d ? d->N : one.N;
@@ -278,10 +310,16 @@ __global__ void __launch_bounds__(kQuadWarps * 32, NP <= 8 ? 12 : (NP <= 12 ? 9 
         const uint32_t cnt = min(left, (uint32_t)GjQuad<NP>::BLOCKS);
         const uintptr_t at = reinterpret_cast<uintptr_t>(S) | reinterpret_cast<uintptr_t>(P);
         const uint32_t vw = (n % 4 == 0 && (at & 15u) == 0) ? 4u : ((n % 2 == 0 && (at & 7u) == 0) ? 2u : 1u);
-        invert_quads<NP>(S + (size_t)k * 3 * n * n + (size_t)n * n, P + (size_t)k * (tri_layout ? 3 : 1) * n * n, n, cnt,
-                         tri_layout, vw, scratch[warp], lane);
+        ok &= invert_quads<NP>(S + (size_t)k * 3 * n * n + (size_t)n * n, P + (size_t)k * (tri_layout ? 3 : 1) * n * n, n, cnt,
+                               tri_layout, vw, scratch[warp], lane);
         if (cnt == left) ++lo;  // the next knots are the next system's
         gk += cnt;
+    }
+    if (!__all_sync(0xffffffffu, ok)) {
+        static_assert(quad_words<NP>() >= 32 + NP * NP, "scratch of the other inverse");
+        gk = ((uint64_t)blockIdx.x * kQuadWarps + warp) * per;
+        invert_range_any<float, float, float>(sys ? descs : nullptr, sys, knot_prefix, nsys, gk, min(gk + per, total_knots),
+                                                tri_layout, &one, scratch[warp], scratch[warp] + 32);
     }
 }
 
