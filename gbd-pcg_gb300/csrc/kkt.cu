@@ -21,13 +21,12 @@
 // written in the cbtd layout (padding blocks of knots 0 and N-1 zero), gamma
 // and lambda are n N, x is n (N+1), u is m N.
 //
-// Both kernels run one warp per knot and read each input once and write each
-// output once, so HBM bandwidth bounds them.  The formation stages [A_k | B_k]
-// in shared memory and forms its Gram product as a register tile per lane;
-// S_kk is symmetrised through shared memory (0.5 (S + S^T), exactly
-// symmetric), and the formation can invert S_kk in the same warp (the
-// block-Jacobi Phi^-1).  In the back-substitution lane l reads column l of
-// [A_k | B_k].
+// Both kernels read each input once and write each output once; a warp takes one to
+// four knots.  The formation stages [A_k | B_k] in shared memory and forms its Gram
+// product as a register tile per lane; S_kk is symmetrised through shared memory
+// (0.5 (S + S^T), exactly symmetric), and the formation can invert S_kk in the same
+// warp (the block-Jacobi Phi^-1).  In the back-substitution a lane reads a column of
+// [A_k | B_k].  What bounds each stands at the kernels.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -44,8 +43,8 @@ void set_last_error(const std::string &msg);
 namespace {
 
 constexpr int kKktMaxN = 32;  // n, m <= 32
-// knots per CTA (4 float, 2 double: at most about 40 KB of dynamic shared
-// memory either way in the formation)
+// warps per CTA (4 float, 2 double: at most 40 KB of dynamic shared memory either
+// way in the formation, at n = m = 32)
 template <typename T>
 constexpr int kkt_warps() { return sizeof(T) == 8 ? 2 : 4; }
 
@@ -54,8 +53,8 @@ constexpr int kkt_warps() { return sizeof(T) == 8 ? 2 : 4; }
 // or of B_k, contiguous in global memory; rows are NP + 4 elements (a 16-byte
 // multiple), rows n..NP-1 zero.  X, the Gram product, takes Mt's place.  d, d w
 // (L = n + m each) and Qi_{k+1} follow, then (with the fused inverse) the
-// symmetrised S_kk of every knot the warp inverts at once, Y[c][r] with rows of
-// NP + 4, and the scratch of the inverse.
+// symmetrised S_kk of every knot the warp inverts at once, if several, Y[c][r] with
+// rows of NP + 4, and the scratch of the inverse.
 template <int NP>
 __host__ __device__ constexpr uint32_t schur_ldt() { return NP + 4; }
 // knots a warp inverts at once
@@ -63,14 +62,14 @@ template <int NP>
 __host__ __device__ constexpr uint32_t schur_knots() { return 32 / gbdpcg::gj_lanes(NP); }
 
 template <int NP>
-__host__ __device__ inline uint32_t schur_mt_elems(uint32_t L) {
+__host__ __device__ constexpr uint32_t schur_mt_elems(uint32_t L) {
     const uint32_t mt = L * schur_ldt<NP>(), x = (NP * (NP + 1) + 3) & ~3u;
     return mt > x ? mt : x;
 }
 template <int NP, bool PINV>
-__host__ __device__ inline uint32_t schur_warp_elems(uint32_t L) {
+__host__ __device__ constexpr uint32_t schur_warp_elems(uint32_t L) {
     return schur_mt_elems<NP>(L) + 2 * ((L + 3) & ~3u) + 32 +
-           (PINV ? schur_knots<NP>() * NP * schur_ldt<NP>() + gbdpcg::kGjElems : 0);
+           (PINV ? (schur_knots<NP>() > 1 ? schur_knots<NP>() * NP * schur_ldt<NP>() : 0) + gbdpcg::kGjElems : 0);
 }
 
 // Asynchronous copy of VW consecutive elements global -> shared (cp.async, no
@@ -183,13 +182,25 @@ __device__ __forceinline__ void gram_tile(const T *Mt, uint32_t ldt, const T *dv
 //
 // What bounds it: instruction issue and the shared-memory pipe (n=24, m=12: 5930
 // instructions a knot with one element an access, one row an FMA and a select an
-// element of the inverse; now 4200, the pipe 71% busy).  The register caps keep 28
-// warps on an SM (n=24 with Phi^-1 at 96 registers: 365 us).  Measured, us, before
-// and now, N=65536 FP32: n=24 m=12 212 -> 183, with Phi^-1 382 -> 329; n=14 m=7
+// element of the inverse; now 4200, the pipe 71% busy).  Measured, us, before
+// and now, N=65536 FP32: n=24 m=12 212 -> 183, with Phi^-1 382 -> 322; n=14 m=7
 // 114 -> 102, 198 -> 140; n=6 m=3 with Phi^-1 96 -> 56.  FP64 is bound by the FP64
-// pipe (n=14 m=7 N=30000 with Phi^-1 1365 -> 980).
+// pipe (n=14 m=7 N=30000 with Phi^-1 1365 -> 862), so it takes 16-byte accesses only
+// with Phi^-1 (n=24 m=12 N=4096 without 274 us, 243 with 8 bytes; with Phi^-1 422
+// and 475).
+//
+// CTAs an SM that the registers allow: as many as hide the latency of a knot's
+// stages.  FP32 n=31 m=15 with five and its S_kk stored twice 327 us, with Phi^-1
+// 631; now 310 and 561; n=32 m=32 with Phi^-1 688 -> 580; n=3 m=1 40 -> 34; FP64
+// n=24 m=12 N=4096 with six 274 us, now 241.
+template <typename T, int NP, bool PINV>
+constexpr int schur_ctas() {
+    if (sizeof(T) == 8) return 8;
+    if (PINV) return NP <= 24 ? 7 : 6;
+    return NP <= 8 ? 12 : (NP <= 24 ? 7 : 8);
+}
 template <typename T, int NP, int W, bool PINV, int VW>
-__global__ void __launch_bounds__(W * 32, sizeof(T) == 4 ? (NP <= 24 ? 7 : 5) : 6)
+__global__ void __launch_bounds__(W * 32, schur_ctas<T, NP, PINV>())
     form_schur_kernel(const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ Qd,
                       const T *__restrict__ Rd, const T *__restrict__ q, const T *__restrict__ r,
                       const T *__restrict__ c, uint32_t n, uint32_t m, uint32_t N, uint32_t kw, T *__restrict__ S,
@@ -202,7 +213,7 @@ __global__ void __launch_bounds__(W * 32, sizeof(T) == 4 ? (NP <= 24 ? 7 : 5) : 
     if (k0 >= N) return;  // warp-uniform; no CTA barrier below
     const uint32_t L = n + m, L4 = (L + 3) & ~3u, nn = n * n;
     T *Mt = reinterpret_cast<T *>(schur_smem) + (size_t)warp * schur_warp_elems<NP, PINV>(L);
-    T *X = Mt, *dv = Mt + schur_mt_elems<NP>(L), *dw = dv + L4, *qn = dw + L4, *Y = qn + 32, *s = Y + KW * NP * ldt;
+    T *X = Mt, *dv = Mt + schur_mt_elems<NP>(L), *dw = dv + L4, *qn = dw + L4, *Y = qn + 32, *s = Y + (PINV && KW > 1 ? KW * NP * ldt : 0);
     // pieces of VW elements: n / VW in a column; x / cv = (x magic) >> 16 for x < 2048
     const uint32_t cv = n / VW, magic = (65536u + cv - 1) / cv;
     const uint32_t kend = min(k0 + kw, N);
@@ -284,7 +295,7 @@ __global__ void __launch_bounds__(W * 32, sizeof(T) == 4 ? (NP <= 24 ? 7 : 5) : 
 #pragma unroll
             for (int u = 0; u < VW; ++u) v[u] = T(0.5) * (X[(p + u) * xs + col] + X[col * xs + p + u]);
             store_vec<T, VW>(Sk + nn + e * VW, v);
-            if constexpr (PINV) store_vec<T, VW>(Yk + col * ldt + p, v);
+            if constexpr (PINV && KW > 1) store_vec<T, VW>(Yk + col * ldt + p, v);
         }
         __syncwarp();  // X is free for the next knot's columns, Y complete
     }
@@ -293,22 +304,30 @@ __global__ void __launch_bounds__(W * 32, sizeof(T) == 4 ? (NP <= 24 ? 7 : 5) : 
         // (the values just written), identity beyond n
         const uint32_t g = lane / GL, rr = lane % GL;
         const bool mine = k0 + g < kend && rr < n;
-        const T *Yg = Y + g * NP * ldt;
+        T *Yg = KW > 1 ? Y + g * NP * ldt : X;
         T a[NP];
 #pragma unroll
-        for (int cc = 0; cc < NP; ++cc)
-            a[cc] = (mine && (uint32_t)cc < n) ? Yg[cc * ldt + rr] : ((uint32_t)cc == rr ? T(1) : T(0));
-        const T diag = mine ? Yg[rr * ldt + rr] : T(1);
+        for (int cc = 0; cc < NP; ++cc) {
+            a[cc] = (uint32_t)cc == rr ? T(1) : T(0);
+            if (mine && (uint32_t)cc < n) a[cc] = KW > 1 ? Yg[cc * ldt + rr] : T(0.5) * (Yg[rr * xs + cc] + Yg[cc * xs + rr]);
+        }
+        const T diag = mine ? Yg[rr * (KW > 1 ? ldt : xs) + rr] : T(1);
         T *sg = s + g * 3 * GL;
         bool ok;
         const T h = T(0.5) * gbdpcg::gj_inverse<T, NP, GL>(a, diag, mine, sg, rr, ok);  // ends with a warp sync: Y is free
         if (!__all_sync(0xffffffffu, ok)) {
-            for (uint32_t k = k0; k < kend; ++k)
-                gbdpcg::gj_invert_any(Y + (k - k0) * NP * ldt, ldt, Pinv + (size_t)k * nn, false, n, s, lane);
+            if constexpr (KW > 1) {
+                for (uint32_t k = k0; k < kend; ++k)
+                    gbdpcg::gj_invert_any(Y + (k - k0) * NP * ldt, ldt, Pinv + (size_t)k * nn, false, n, s, lane);
+            } else {
+                for (uint32_t cc = 0; lane < n && cc < lane; ++cc)
+                    X[lane * xs + cc] = X[cc * xs + lane] = T(0.5) * (X[lane * xs + cc] + X[cc * xs + lane]);
+                gbdpcg::gj_invert_any(X, xs, Pinv + (size_t)k0 * nn, false, n, s, lane);
+            }
             return;
         }
         const T *D = sg + 2 * GL;
-        T *Xg = Y + g * NP * ldt;
+        T *Xg = Yg;
         if (rr < (uint32_t)NP) {
 #pragma unroll
             for (int cc = 0; cc < NP; ++cc) Xg[rr * xs + cc] = a[cc];
@@ -324,9 +343,10 @@ __global__ void __launch_bounds__(W * 32, sizeof(T) == 4 ? (NP <= 24 ? 7 : 5) : 
 }
 
 // s + sum_j col[j] w[j], j ascending, VW elements an access (n a multiple of VW,
-// both addresses aligned to it).
-template <typename T, int VW>
+// both addresses aligned to it), U accesses an iteration.
+template <typename T, int VW, int U>
 __device__ __forceinline__ T col_dot(const T *col, const T *w, uint32_t n, T s) {
+#pragma unroll U
     for (uint32_t j = 0; j < n; j += VW) {
         T a[VW], b[VW];
         load_vec<T, VW>(col + j, a);
@@ -343,19 +363,26 @@ __device__ __forceinline__ T col_dot(const T *col, const T *w, uint32_t n, T s) 
 // the columns of A_k go first, then those of B_k: together their lines outgrow the
 // L1 of an SM's 64 warps (n=24 m=12: 55 us against 50; n=24 m=8 46 / 44, n=16 m=8
 // 31.3 / 32.0).  A lane reads its own
-// contiguous column with accesses of 16 or 8 bytes where n and the addresses allow.
+// contiguous column with accesses of 16 or 8 bytes where n and the addresses allow,
+// U an iteration: one where every lane has a column to read, four where the lanes
+// beyond the block's columns wait (TWO) or an access is 4 bytes.
 //
 // What bounds it: HBM and, for short columns, the L1 requests (a column is 24 to
 // 128 bytes).  Measured, us, before (one pass for A_k, one for B_k, one element an
-// access unless n is a multiple of 4) and now: n=14 m=7 N=40001 22.9 -> 19.7, n=6
-// m=3 N=60000 21.1 -> 10.4, n=13 m=6 N=60000 30.7 -> 25.3, n=22 m=11 N=60000 56.3 ->
-// 42.4; n=24 m=12 N=65536 (50.4) and FP64, bound by its pipe, are as they were.
+// access unless n is a multiple of 4) and now, one problem again and again (n=14: its
+// 70 MB lie in the L2) / eight problems in turn (n=6: in the L2 still): n=14
+// m=7 N=60000 27.6 -> 19.7 / 31.6 -> 25.7, n=6 m=3 21.3 -> 9.8 / 27.0 -> 9.8, n=12
+// m=6 19.2 -> 14.9 / 27.4 -> 18.8, n=13 m=6 25.2 -> 23.7 / 30.3 -> 27.4, n=22 m=11
+// 56.1 -> 45.7 / 55.8 -> 45.1; FP64 n=14 m=7 N=30000 81.8 -> 60.4 / 82.4 -> 62.0.
+// n=24 m=12 (47.5 -> 44.2) and FP64 of 25 columns or more, bound by its pipe, are
+// as they were.
 template <typename T, int GL, int VW, bool TWO, int kKktWarps>
 __global__ void __launch_bounds__(kKktWarps * 32)
     kkt_backsub_kernel(const T *__restrict__ A, const T *__restrict__ B, const T *__restrict__ Qd,
                        const T *__restrict__ Rd, const T *__restrict__ q, const T *__restrict__ r,
                        const T *__restrict__ lambda, uint32_t n, uint32_t m, uint32_t N, T *__restrict__ x,
                        T *__restrict__ u) {
+    constexpr int U = TWO || (sizeof(T) == 4 && VW == 1) ? 4 : 1;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t k = (blockIdx.x * kKktWarps + (threadIdx.x >> 5)) * (32 / GL) + lane / GL;
     if (k > N) return;  // knots 0..N (x) and 0..N-1 (u)
@@ -364,12 +391,12 @@ __global__ void __launch_bounds__(kKktWarps * 32)
         const uint32_t l = lane;
         if (l < n) {
             T s = q[(size_t)k * n + l];
-            if (k < N) s = col_dot<T, VW>(A + ((size_t)k * n + l) * n, lk, n, s);
+            if (k < N) s = col_dot<T, VW, U>(A + ((size_t)k * n + l) * n, lk, n, s);
             if (k > 0) s -= lambda[(size_t)(k - 1) * n + l];
             x[(size_t)k * n + l] = -s / Qd[(size_t)k * n + l];
         }
         if (k < N && l < m) {
-            const T s = col_dot<T, VW>(B + ((size_t)k * m + l) * n, lk, n, r[(size_t)k * m + l]);
+            const T s = col_dot<T, VW, U>(B + ((size_t)k * m + l) * n, lk, n, r[(size_t)k * m + l]);
             u[(size_t)k * m + l] = -s / Rd[(size_t)k * m + l];
         }
         return;
@@ -379,7 +406,7 @@ __global__ void __launch_bounds__(kKktWarps * 32)
         T s = is_x ? q[e] : r[e];
         const T d = is_x ? Qd[e] : Rd[e];
         if (k < N)  // + (A_k^T lambda_k)_i = sum_j A_k[j][i] lambda_k[j], B_k^T lambda_k alike
-            s = col_dot<T, VW>(is_x ? A + ((size_t)k * n + l) * n : B + ((size_t)k * m + (l - n)) * n, lk, n, s);
+            s = col_dot<T, VW, U>(is_x ? A + ((size_t)k * n + l) * n : B + ((size_t)k * m + (l - n)) * n, lk, n, s);
         if (is_x) {
             if (k > 0) s -= lambda[(size_t)(k - 1) * n + l];
             x[e] = -s / d;
@@ -422,10 +449,11 @@ int form_schur(const T *A, const T *B, const T *Qd, const T *Rd, const T *q, con
     int rc = check(p, 9, n, m, N);
     if (rc) return rc;
     constexpr int W = kkt_warps<T>();
-    // elements of an access: what n and the blocks' addresses allow
+    // elements of an access: what n and the blocks' addresses allow (FP64 without
+    // Phi^-1: one, see the kernel)
     const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(S);
     constexpr uint32_t V16 = 16 / sizeof(T);
-    const bool v16 = n % V16 == 0 && (at & 15u) == 0, v8 = sizeof(T) == 4 && n % 2 == 0 && (at & 7u) == 0;
+    const bool v16 = (sizeof(T) == 4 || Pinv) && n % V16 == 0 && (at & 15u) == 0, v8 = sizeof(T) == 4 && n % 2 == 0 && (at & 7u) == 0;
     auto go = [&](auto np) -> int {
         constexpr int NP = decltype(np)::value;
         auto launch = [&](auto kern, size_t smem, uint32_t knots) -> int {
