@@ -21,9 +21,14 @@
 // hands the results to every thread.  All CTAs add the same words in the same
 // order, so they take the same decisions.  Two sets of mailboxes alternate: a
 // CTA posts exchange e + 2 only after it has read every CTA's word of e + 1,
-// which that CTA posted after it had read all of e.  Every wait gives up after
-// about a second and sets the CTA's flag (status TIMEOUT), and every later wait
-// then returns at once.
+// which that CTA posted after it had read all of e.
+//
+// Every wait gives up after about a second (the CTAs start together: beside another
+// solve that held one SM for 2.5 s, the launch waited and no wait ran out).  A CTA
+// that gives up uses none of the words it has and posts none any more: it ends as
+// TIMEOUT, and so does, a wait later, every CTA that needs its next word.  CTA 0,
+// whose status is the solve's, needs a word of every CTA to go on, so it reports
+// another end only if all that was left to do was to stop.
 //
 // Every CTA posts to mailboxes of each receiver's own (152 words a value): with
 // one word a CTA that all poll, 152 SMs queue at the same few lines (3.5 us an
@@ -85,14 +90,14 @@ __device__ __forceinline__ V from_words(uint32_t lo, uint32_t hi) {
     else return __uint_as_float(lo);
 }
 
-// A bounded spin: counts the failed polls and gives up after about a second.
+// A bounded spin: counts the failed polls and gives up after `limit` ns.
 struct SpinLimit {
     uint64_t t0 = 0;
     uint32_t spins = 0;
-    __device__ __forceinline__ bool expired(volatile uint32_t *timed_out) {
+    __device__ __forceinline__ bool expired(volatile uint32_t *timed_out, uint64_t limit) {
         if (*timed_out) return true;
         if (spins == 0) t0 = global_ns();
-        if ((++spins & 63u) == 0 && global_ns() - t0 > 1000000000ull) *timed_out = 1u;
+        if ((++spins & 63u) == 0 && global_ns() - t0 > limit) *timed_out = 1u;
         return *timed_out != 0;
     }
 };
@@ -110,12 +115,14 @@ struct GridOut {
 // thread of every CTA), and, with `halos`, the neighbours' boundary values
 // posted for this exchange, from the left into hl and from the right into hr.
 // fin(q, sum, out): run by the warp that added value q (quotient, exit tests).
-template <typename T, typename A, int NP, int NQ, typename F>
-__device__ __forceinline__ void grid_exchange(A (&v)[NQ], A *part, GridOut<T, A> *out, const GridParams &gp, uint32_t &seq,
+// Returns whether it is complete.
+template <typename T, typename A, int NP, bool PROBE, int NQ, typename F>
+__device__ __forceinline__ bool grid_exchange(A (&v)[NQ], A *part, GridOut<T, A> *out, const GridParams &gp, uint32_t &seq,
                                               uint32_t C, uint32_t rank, uint32_t n, bool halos, T *hl, T *hr, F &&fin) {
     constexpr int NW = sizeof(A) / 4, TW = sizeof(T) / 4;
     constexpr uint32_t kHaloWords = 2 * NP;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const uint64_t limit = PROBE ? gp.probe_limit_ns : 1000000000ull;
     ++seq;
     const uint32_t buf = seq & 1u;
     // [receiver][word][sender]: every CTA polls lines of its own
@@ -156,7 +163,7 @@ __device__ __forceinline__ void grid_exchange(A (&v)[NQ], A *part, GridOut<T, A>
 #pragma unroll
             for (uint32_t u = 0; u < kGridMaxCtas / 32; ++u) {
                 const uint32_t to = u * 32 + lane;
-                if (to < C) {
+                if (to < C && !(PROBE && seq == gp.probe_seq && rank == gp.probe_from && to == gp.probe_to)) {
 #pragma unroll
                     for (int k = 0; k < NW; ++k)
                         mail_post(sums + ((size_t)to * kGridWords + job * 2 + k) * C + rank, seq, word_of(t[0], k));
@@ -184,7 +191,7 @@ __device__ __forceinline__ void grid_exchange(A (&v)[NQ], A *part, GridOut<T, A>
                     }
                 }
                 if (__all_sync(0xffffffffu, ok)) break;
-                const bool late = spin.expired(&out->timed_out);
+                const bool late = spin.expired(&out->timed_out, limit);
                 if (__any_sync(0xffffffffu, late)) break;
             }
             A s[1] = {A(0)};
@@ -203,7 +210,7 @@ __device__ __forceinline__ void grid_exchange(A (&v)[NQ], A *part, GridOut<T, A>
                 for (uint32_t e = lane; e < n * TW; e += 32) {
                     uint64_t w = mail_peek(in + e);
                     while ((uint32_t)(w >> 32) != seq) {
-                        if (spin.expired(&out->timed_out)) break;
+                        if (spin.expired(&out->timed_out, limit)) break;
                         w = mail_peek(in + e);
                     }
                     dst[e] = (uint32_t)w;
@@ -215,6 +222,7 @@ __device__ __forceinline__ void grid_exchange(A (&v)[NQ], A *part, GridOut<T, A>
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < NQ; ++q) v[q] = out->sum[q];
+    return out->timed_out == 0u;
 }
 
 // Posts row i's boundary value for the next exchange into neighbour `to`'s
@@ -273,7 +281,9 @@ __device__ __forceinline__ T grid_row(const T *__restrict__ M, int b0, int b1, c
 // G: rows per thread (thread t owns rows t, t + blockDim.x, ... of its CTA).
 // REG: the rows of S are held in registers for the whole solve (G = 1); else
 // they are read in every product, like Phi^-1 always.
-template <typename T, typename A, int NP, bool PTRI, int G, bool REG>
+// PROBE: the wait limit is the launch's, and one sum of one exchange is not posted
+// (gbdpcg_probe_grid_timeout).
+template <typename T, typename A, int NP, bool PTRI, int G, bool REG, bool PROBE = false>
 __global__ void __launch_bounds__(grid_threads<T, NP, REG>(), 1) pcg_grid_kernel(const GridParams gp) {
     static_assert(!REG || G == 1, "one row a thread in registers");
     using Plan = SmemPlanGrid<T, A, NP, PTRI>;
@@ -366,6 +376,7 @@ __global__ void __launch_bounds__(grid_threads<T, NP, REG>(), 1) pcg_grid_kernel
     // ---- r = gamma - S lambda0   (include/pcg.cuh:119-126)
     T lam[G], r[G], p[G], z[G], y[G];
     A gg;
+    bool alive;
     {
         if (lam0) {
 #pragma unroll
@@ -388,13 +399,13 @@ __global__ void __launch_bounds__(grid_threads<T, NP, REG>(), 1) pcg_grid_kernel
             if (act[g]) vr[(lk[g] + 1) * NP + ri[g]] = r[g];
             if constexpr (PTRI) post(g, r[g]);
         }
-        grid_exchange<T, A, NP, 1>(v1, part, out, gp, seq, C, rank, n, PTRI, vr, vr + (nk + 1) * NP,
-                                   [](int, A, GridOut<T, A> *, uint32_t) {});
+        alive = grid_exchange<T, A, NP, PROBE, 1>(v1, part, out, gp, seq, C, rank, n, PTRI, vr, vr + (nk + 1) * NP,
+                                                  [](int, A, GridOut<T, A> *, uint32_t) {});
         gg = v1[0];
     }
     // ---- z = Phi^-1 r; p = z; eta = r.z   (include/pcg.cuh:131-149)
-    A eta;
-    {
+    A eta = A(0);
+    if (alive) {
         A v1[1] = {A(0)};
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -404,17 +415,17 @@ __global__ void __launch_bounds__(grid_threads<T, NP, REG>(), 1) pcg_grid_kernel
             post(g, z[g]);
             acc_madd(v1[0], r[g], z[g]);
         }
-        grid_exchange<T, A, NP, 1>(v1, part, out, gp, seq, C, rank, n, true, vp, vp + (nk + 1) * NP,
-                                   [](int, A, GridOut<T, A> *, uint32_t) {});
+        alive = grid_exchange<T, A, NP, PROBE, 1>(v1, part, out, gp, seq, C, rank, n, true, vp, vp + (nk + 1) * NP,
+                                                  [](int, A, GridOut<T, A> *, uint32_t) {});
         eta = v1[0];
     }
     const A thr = A(d.tol * d.tol * (double)gg), tol = A(d.tol);
 
     // ---- main loop   (include/pcg.cuh:154-208)
     uint32_t iter = 0;
-    int32_t status = ST_MAX_ITER;
+    int32_t status = alive ? ST_MAX_ITER : ST_TIMEOUT;
     A eta_new = A(0), rr = A(0);
-    const uint32_t max_iter = d.max_iter;
+    const uint32_t max_iter = alive ? d.max_iter : 0u;
     for (; iter < max_iter;) {
         uint32_t bad;
         {
@@ -425,15 +436,16 @@ __global__ void __launch_bounds__(grid_threads<T, NP, REG>(), 1) pcg_grid_kernel
                 if constexpr (PTRI) post(g, y[g]);  // the neighbours' r halo
                 acc_madd(v1[0], p[g], y[g]);
             }
-            grid_exchange<T, A, NP, 1>(v1, part, out, gp, seq, C, rank, n, PTRI, uh, uh + NP,
-                                       [&](int, A s, GridOut<T, A> *o, uint32_t lane) {
-                                           const T a = (s == A(0)) ? T(0) : acc_ratio<T>(eta, s);
-                                           if (lane == 0) {
-                                               o->ratio = a;
-                                               o->code[0] = acc_finite(s) ? 0u : kNotFinite;
-                                           }
-                                       });
+            alive = grid_exchange<T, A, NP, PROBE, 1>(v1, part, out, gp, seq, C, rank, n, PTRI, uh, uh + NP,
+                                                      [&](int, A s, GridOut<T, A> *o, uint32_t lane) {
+                                                          const T a = (s == A(0)) ? T(0) : acc_ratio<T>(eta, s);
+                                                          if (lane == 0) {
+                                                              o->ratio = a;
+                                                              o->code[0] = acc_finite(s) ? 0u : kNotFinite;
+                                                          }
+                                                      });
         }
+        if (!alive) { status = ST_TIMEOUT; break; }
         const T alpha = out->ratio;
         bad = out->code[0];
 #pragma unroll
@@ -453,26 +465,26 @@ __global__ void __launch_bounds__(grid_threads<T, NP, REG>(), 1) pcg_grid_kernel
                 acc_madd(v2[0], r[g], z[g]);
                 if (relres) acc_madd(v2[1], r[g], r[g]);
             }
-            grid_exchange<T, A, NP, 2>(v2, part, out, gp, seq, C, rank, n, true, zh, zh + NP,
-                                       [&](int q, A s, GridOut<T, A> *o, uint32_t lane) {
-                                           if (q == 0) {
-                                               const T b = acc_ratio<T>(s, eta);
-                                               if (lane == 0) {
-                                                   o->ratio = b;
-                                                   o->code[0] = (acc_finite(s) ? 0u : kNotFinite) |
-                                                                (acc_abs(s) < tol ? kExitTest : 0u);
-                                               }
-                                           } else if (lane == 0) {
-                                               o->code[1] = s <= thr ? kExitTest : 0u;
-                                           }
-                                       });
+            alive = grid_exchange<T, A, NP, PROBE, 2>(v2, part, out, gp, seq, C, rank, n, true, zh, zh + NP,
+                                                      [&](int q, A s, GridOut<T, A> *o, uint32_t lane) {
+                                                          if (q == 0) {
+                                                              const T b = acc_ratio<T>(s, eta);
+                                                              if (lane == 0) {
+                                                                  o->ratio = b;
+                                                                  o->code[0] = (acc_finite(s) ? 0u : kNotFinite) |
+                                                                               (acc_abs(s) < tol ? kExitTest : 0u);
+                                                              }
+                                                          } else if (lane == 0) {
+                                                              o->code[1] = s <= thr ? kExitTest : 0u;
+                                                          }
+                                                      });
             eta_new = v2[0];
             rr = v2[1];
         }
         ++iter;
         const T beta = out->ratio;
         bad |= out->code[0] & kNotFinite;
-        if (out->timed_out) { status = ST_TIMEOUT; break; }
+        if (!alive) { status = ST_TIMEOUT; break; }
         if (bad) { status = ST_BREAKDOWN; break; }
         if (out->code[relres ? 1 : 0] & kExitTest) { status = ST_CONVERGED; break; }
         eta = eta_new;

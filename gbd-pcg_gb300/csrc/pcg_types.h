@@ -110,7 +110,10 @@ struct GridParams {
     uint64_t *sums;   // [2][C receivers][kGridWords][C senders] mailboxes of the reduced values
     uint64_t *halos;  // [2][C][2 sides][2 NP] mailboxes of the boundary values
     uint32_t kmax;    // knots per CTA
-    uint32_t pad_;
+    // PROBE kernels: the limit of every wait, and the sum that is not posted, from CTA
+    // probe_from to probe_to in exchange probe_seq (1, 2, ..)
+    uint32_t probe_seq, probe_from, probe_to;
+    uint64_t probe_limit_ns;
 };
 constexpr uint32_t kGridWords = 2 * 2;    // two values of up to two 32-bit words
 constexpr uint32_t kGridMaxCtas = 160;    // CTAs whose words a warp polls (5 a lane)

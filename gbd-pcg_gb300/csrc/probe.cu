@@ -21,6 +21,7 @@
 
 #include "../../include/gbdpcg.h"
 #include "pcg_cluster.cuh"
+#include "pcg_grid.cuh"
 
 namespace gbdpcg {
 void set_last_error(const std::string &msg);
@@ -284,6 +285,79 @@ int gbdpcg_probe_timeout(int device, uint32_t cluster, int *status, double *wait
     for (int x : st)
         if (x != GBDPCG_TIMEOUT) worst = x;  // a CTA whose wait did not give up
     *status = worst;
+    *waited_ms = (double)ms;
+    return GBDPCG_SUCCESS;
+}
+
+int gbdpcg_probe_grid_timeout(int device, uint32_t exchange, int *status, double *waited_ms) {
+    if (!status || !waited_ms) return probe_fail(GBDPCG_ERR_INVALID_ARGUMENT, "NULL pointer");
+    constexpr uint32_t n = 14, N = 8, C = 4, K = 2, threads = 128, passes = 6;
+    if (exchange > 2 + 2 * passes) return probe_fail(GBDPCG_ERR_INVALID_ARGUMENT, "exchange 0..14");
+    int prev = -1;
+    cudaGetDevice(&prev);
+    if (prev != device && cudaSetDevice(device) != cudaSuccess)
+        return probe_fail(GBDPCG_ERR_INVALID_ARGUMENT, "bad device");
+    // S = tridiag(-1, 2 + j / n, -1) between the knots, entry by entry j; Phi^-1 = 1
+    std::vector<float> S(3 * n * n * N, 0.f), P(n * n * N, 0.f), v(n * N);
+    for (uint32_t k = 0; k < N; ++k)
+        for (uint32_t j = 0; j < n; ++j) {
+            float *d = S.data() + (size_t)k * 3 * n * n + j * n + j;
+            if (k > 0) d[0] = -1.f;
+            d[n * n] = 2.f + (float)j / n;
+            if (k + 1 < N) d[2 * n * n] = -1.f;
+            P[(size_t)k * n * n + j * n + j] = 1.f;
+            v[k * n + j] = 1.f + (float)((k * n + j) % 5);
+        }
+    const size_t sums = (size_t)2 * kGridWords * C * C * 8, halos = (size_t)2 * C * 2 * 2 * n * 8;
+    const size_t at_S = sums + halos, at_P = at_S + S.size() * 4, at_v = at_P + P.size() * 4, at_l = at_v + v.size() * 4,
+                 at_r = at_l + v.size() * 4, total = at_r + sizeof(SysResult);
+    char *d = nullptr;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    SysResult res;
+    memset(&res, 0, sizeof(res));
+    res.status = -2;
+    float ms = 0.f;
+    cudaError_t e = cudaMalloc(&d, total);
+    if (e == cudaSuccess) e = cudaMemset(d, 0, total);
+    if (e == cudaSuccess) e = cudaMemcpy(d + at_S, S.data(), S.size() * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + at_P, P.data(), P.size() * 4, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + at_v, v.data(), v.size() * 4, cudaMemcpyHostToDevice);
+    GridParams gp;
+    memset(&gp, 0, sizeof(gp));
+    gp.one.S = d + at_S;
+    gp.one.P = d + at_P;
+    gp.one.gamma = d + at_v;
+    gp.one.lambda = d + at_l;
+    gp.one.n = n;
+    gp.one.N = N;
+    gp.one.max_iter = passes;
+    gp.one.flags = SYS_EXIT_RELRES | SYS_LAMBDA0_ZERO;
+    gp.result = reinterpret_cast<SysResult *>(d + at_r);
+    gp.sums = reinterpret_cast<uint64_t *>(d);
+    gp.halos = gp.sums + sums / 8;
+    gp.kmax = K;
+    gp.probe_seq = exchange;
+    gp.probe_from = 2;
+    gp.probe_to = 1;
+    gp.probe_limit_ns = 20000000ull;
+    void *args[] = {&gp};
+    const void *func = (const void *)&pcg_grid_kernel<float, float, n, false, 1, true, true>;
+    if (e == cudaSuccess) e = cudaEventCreate(&e0);
+    if (e == cudaSuccess) e = cudaEventCreate(&e1);
+    if (e == cudaSuccess) e = cudaEventRecord(e0, 0);
+    if (e == cudaSuccess)
+        e = cudaLaunchCooperativeKernel(func, dim3(C), dim3(threads), args,
+                                        SmemPlanGrid<float, float, n, false>::bytes(K, C, threads / 32), 0);
+    if (e == cudaSuccess) e = cudaEventRecord(e1, 0);
+    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+    if (e == cudaSuccess) e = cudaMemcpy(&res, d + at_r, sizeof(res), cudaMemcpyDeviceToHost);
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+    if (d) cudaFree(d);
+    if (prev >= 0 && prev != device) cudaSetDevice(prev);
+    if (e != cudaSuccess) return probe_fail(GBDPCG_ERR_CUDA, std::string("grid timeout probe: ") + cudaGetErrorString(e));
+    *status = res.status;
     *waited_ms = (double)ms;
     return GBDPCG_SUCCESS;
 }

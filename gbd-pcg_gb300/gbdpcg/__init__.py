@@ -103,6 +103,14 @@ def probe_timeout(device=0, cluster=2) -> tuple:
     return st.value, ms.value
 
 
+def probe_grid_timeout(device=0, exchange=0) -> tuple:
+    """A whole-GPU solve one of whose CTAs misses a word of the given exchange
+    (gbdpcg_probe_grid_timeout): (status of the solve, ms)."""
+    st, ms = ctypes.c_int(0), ctypes.c_double(0)
+    _check(lib().gbdpcg_probe_grid_timeout(device, exchange, ctypes.byref(st), ctypes.byref(ms)), "gbdpcg_probe_grid_timeout")
+    return st.value, ms.value
+
+
 class System(ctypes.Structure):
     _fields_ = [("S", ctypes.c_void_p), ("Pinv", ctypes.c_void_p), ("gamma", ctypes.c_void_p),
                 ("lambda_", ctypes.c_void_p), ("lambda_fwd", ctypes.c_void_p), ("dS", ctypes.c_void_p),
@@ -145,6 +153,7 @@ _SIGS = {
     "gbdpcg_plan_timeline_read": ([_P, _P, _U, _P, _P, _U, _P, _P], _I),
     "gbdpcg_probe_primitives": ([_I, _U, _U, _U, _U, _P], _I),
     "gbdpcg_probe_timeout": ([_I, _U, _P, _P], _I),
+    "gbdpcg_probe_grid_timeout": ([_I, _U, _P, _P], _I),
     "gbdpcg_partition": ([_P, _P, _P, _U, _U, _P, _P], _I),
     "gbdpcg_form_schur_f32": ([_P] * 7 + [_U, _U, _U, _P, _P, _P], _I),
     "gbdpcg_form_schur_f64": ([_P] * 7 + [_U, _U, _U, _P, _P, _P], _I),

@@ -489,6 +489,14 @@ GBDPCG_API int gbdpcg_probe_primitives(int device, uint32_t cluster, uint32_t th
  * duration.  The context stays usable.  Synchronous; allocates `cluster`
  * words of device memory. */
 GBDPCG_API int gbdpcg_probe_timeout(int device, uint32_t cluster, int *status, double *waited_ms);
+/* The same for the whole-GPU kernel of one long system: four CTAs solve a small
+ * system for six passes, 14 exchanges, with waits of 20 ms, and in exchange
+ * `exchange` (1, 2, ..; 0: none) CTA 2 does not send its sum to CTA 1, whose wait
+ * then gives up, and after it the others', which need CTA 1's next word.  *status =
+ * the solve's: GBDPCG_TIMEOUT, or GBDPCG_MAX_ITER where the exchange is 0 or the
+ * last one, after which the CTAs only stop.  Synchronous; allocates some KB of
+ * device memory. */
+GBDPCG_API int gbdpcg_probe_grid_timeout(int device, uint32_t exchange, int *status, double *waited_ms);
 /* Waits for the stream and copies the last execution's records (one per
  * system of the cluster launches, grouped by launch; at most `capacity`) and
  * the SM of each CTA (launch 0's CTAs first, in grid order; at most
