@@ -24,6 +24,7 @@
 #include <string>
 
 #include "../../include/gbdpcg.h"
+#include "launch_attr.h"
 
 namespace gbdpcg {
 void set_last_error(const std::string &msg);
@@ -126,7 +127,7 @@ int csr_to_cbtd(const uint32_t *d_row_ptr, const uint32_t *d_col_ind, const T *d
     if (n <= 32) {
         const size_t smem = csr_smem_bytes<T>(n);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(csr_to_cbtd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = gbdpcg::allow_dynamic_smem((const void *)&csr_to_cbtd_kernel<T>, smem);
         if (e == cudaSuccess) {
             csr_to_cbtd_kernel<T><<<(N + kCsrWarps - 1) / kCsrWarps, kCsrWarps * 32, smem, st>>>(
                 d_row_ptr, d_col_ind, d_val, n, N, d_out, d_err);

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../../include/gbdpcg.h"
+#include "launch_attr.h"
 #include "pcg_types.h"
 #include "pcg_variants.h"
 
@@ -63,7 +64,6 @@ struct VariantInfo {
     KernelVariant v;
     int max_threads = 0;  // from the register budget (cudaFuncAttributes)
     int regs = 0;
-    size_t smem_set = 0;  // max dynamic smem attribute already set
     bool nonportable = false;
 };
 
@@ -155,11 +155,7 @@ VariantInfo *find_variant(Registry *reg, bool f64, int acc, int np, bool ptri, i
 }
 
 int prepare_variant(VariantInfo *vi, size_t smem, uint32_t C) {
-    if (smem > 48 * 1024 && smem > vi->smem_set) {
-        GB_CUDA(cudaFuncSetAttribute(vi->v.func, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-        vi->smem_set = smem;
-    }
+    GB_CUDA(allow_dynamic_smem(vi->v.func, smem));
     if (C > 8 && !vi->nonportable) {
         GB_CUDA(cudaFuncSetAttribute(vi->v.func, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         vi->nonportable = true;
@@ -299,8 +295,7 @@ bool plain_fits(Registry *reg, bool f64, uint32_t n, uint32_t N) {
     const size_t smem = plain_smem_bytes(f64, n, N);
     if (smem > (size_t)reg->max_smem_optin) return false;
     const void *func = plain_kernel_ptr(f64);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (allow_dynamic_smem(func, smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -580,8 +575,7 @@ int launch_plain(gbdpcg_handle_s *h, bool f64, const SysDesc &d, SysResult *d_re
     const size_t smem = plain_smem_bytes(f64, d.n, d.N);
     if (smem > (size_t)h->reg->max_smem_optin)
         return fail(GBDPCG_ERR_UNSUPPORTED, "plain algorithm: block row exceeds shared memory");
-    if (smem > 48 * 1024)
-        GB_CUDA(cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GB_CUDA(allow_dynamic_smem(func, smem));
     int per_sm = 0;
     GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, 64, smem));
     if ((int64_t)per_sm * h->reg->sm_count < (int64_t)d.N)
@@ -695,8 +689,7 @@ int solve_grid(gbdpcg_handle_s *h, bool f64, const SysDesc &d, uint32_t layout, 
             GB_CUDA(cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep));
         }
     }
-    if (smem > 48 * 1024)
-        GB_CUDA(cudaFuncSetAttribute(gv->func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    GB_CUDA(allow_dynamic_smem(gv->func, smem));
     const size_t sums = (size_t)2 * kGridWords * C * C * 8, halos = (size_t)2 * C * 2 * 2 * np * 8;
     void *mail = nullptr;
     if (cudaMallocFromPoolAsync(&mail, sums + halos, h->pool, stream) != cudaSuccess) {

@@ -457,11 +457,10 @@ int form_schur(const T *A, const T *B, const T *Qd, const T *Rd, const T *q, con
     auto go = [&](auto np) -> int {
         constexpr int NP = decltype(np)::value;
         auto launch = [&](auto kern, size_t smem, uint32_t knots) -> int {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) {
-                gbdpcg::set_last_error(std::string("form_schur: ") + cudaGetErrorString(e));
-                return GBDPCG_ERR_CUDA;
-            }
+            // (within the 48 KB that any kernel may have: no launch attribute, which
+            // threads would set under one another)
+            static_assert(W * sizeof(T) * schur_warp_elems<NP, true>(kKktMaxN + (NP < kKktMaxN ? NP : kKktMaxN)) <= 48 * 1024,
+                          "shared memory of the formation");
             // few knots: one a warp, side by side (n=14 N=500: 10.5 us against 11.8
             // with two in turn); as many as a warp inverts at once from the knots
             // on that fill the GPU's warps

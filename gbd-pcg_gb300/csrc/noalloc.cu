@@ -34,6 +34,7 @@
 #include <string>
 
 #include "../../include/gbdpcg.h"
+#include "launch_attr.h"
 #include "pcg_types.h"
 #include "pcg_variants.h"
 
@@ -113,8 +114,7 @@ int gbdpcg_solve_plain_noalloc_f32(const float *d_S, const float *d_Pinv, const 
     const size_t smem = gbdpcg::plain_smem_bytes(false, n, N);
     if (smem > (size_t)smem_optin)
         return noalloc_fail(GBDPCG_ERR_UNSUPPORTED, "block row exceeds shared memory");
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = gbdpcg::allow_dynamic_smem(func, smem);
     int per_sm = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, func, 64, smem);
     if (e != cudaSuccess) return noalloc_fail(GBDPCG_ERR_CUDA, std::string("launch set-up: ") + cudaGetErrorString(e));
