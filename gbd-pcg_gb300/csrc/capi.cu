@@ -1377,21 +1377,24 @@ int plan_create_impl(gbdpcg_handle_t h, int dtype, const gbdpcg_system *systems,
     tune_lock.unlock();
     if ((rc = p->d_descs.ensure(sizeof(SysDesc) * count))) return rc;
     if ((rc = p->d_results.ensure(sizeof(SysResult) * p->nresults))) return rc;
-    // knots before each system; by class: the same, and the systems' indices
+    // knots before each system; ordered by class: the same, and the systems' indices
     if ((rc = p->d_prefix.ensure((2 * sizeof(uint64_t) + sizeof(uint32_t)) * count))) return rc;
     prefix.resize(2 * (size_t)count + (count + 1) / 2);
     uint64_t *cprefix = prefix.data() + count;
     std::vector<uint32_t> csys(count);
     memset(&p->jacobi, 0, sizeof(p->jacobi));
+    uint64_t before = 0;
     for (int c = 0, at = 0; c < 5; ++c) {
         p->jacobi.first[c] = (uint32_t)at;
+        p->jacobi.base[c] = before;
         for (uint32_t i = 0; i < count; ++i) {
             if (jacobi_class(p->descs[i].n) != c) continue;
             csys[at] = i;
-            cprefix[at++] = p->jacobi.knots[c];
-            p->jacobi.knots[c] += p->descs[i].N;
+            cprefix[at++] = before;
+            before += p->descs[i].N;
         }
         p->jacobi.count[c] = (uint32_t)at - p->jacobi.first[c];
+        p->jacobi.knots[c] = before - p->jacobi.base[c];
     }
     memcpy(prefix.data() + 2 * (size_t)count, csys.data(), sizeof(uint32_t) * count);
     p->jacobi.prefix = p->d_prefix.as<uint64_t>() + count;

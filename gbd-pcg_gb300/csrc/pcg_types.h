@@ -92,14 +92,15 @@ struct LaunchParams {
     SysDesc one;
 };
 
-// A batch by the block-size classes of the block-Jacobi builder (n <= 8, 12, 16,
-// 24, 32): device arrays of the systems' indices and of the knots of the class
-// before each, class c's at [first[c], first[c] + count[c]).
+// A batch ordered by the block-size classes of the block-Jacobi builder (n <= 8,
+// 12, 16, 24, 32): device arrays of the systems' indices and of the knots before
+// each in that order; class c's systems at [first[c], first[c] + count[c]), its
+// knots [base[c], base[c] + knots[c]).
 struct JacobiClasses {
     const uint32_t *sys;
     const uint64_t *prefix;
     uint32_t first[5], count[5];
-    uint64_t knots[5];
+    uint64_t base[5], knots[5];
 };
 
 // Parameters of the whole-GPU kernel of one long system (pcg_grid.cuh).  The

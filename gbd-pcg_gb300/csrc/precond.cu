@@ -135,27 +135,29 @@ __device__ __noinline__ void invert_range_any(const SysDesc *descs, const uint32
 
 template <typename TI, typename TO, typename CT>
 __global__ void __launch_bounds__(kPrecWarps * 32, sizeof(CT) == 4 ? 5 : 4)
-    block_jacobi_kernel(const SysDesc *__restrict__ descs, const uint64_t *__restrict__ knot_prefix,
-                        uint32_t nsys, uint64_t total_knots, uint32_t per, int tri_layout, uint32_t classes,
-                        const __grid_constant__ SysDesc one) {
+    block_jacobi_kernel(const SysDesc *__restrict__ descs, const uint32_t *__restrict__ sys,
+                        const uint64_t *__restrict__ knot_prefix, uint32_t nsys, uint64_t first_knot, uint64_t end_knot,
+                        uint32_t per, int tri_layout, const __grid_constant__ SysDesc one) {
     __shared__ CT sX[kPrecWarps][kPrecX];
     __shared__ __align__(16) CT sR[kPrecWarps][kGjElems];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint64_t gk = ((uint64_t)blockIdx.x * kPrecWarps + warp) * per;
-    if (gk >= total_knots) return;  // warp-uniform; no CTA-wide barrier below
-    const uint64_t end = min(gk + per, total_knots);
+    const uint64_t start = first_knot + ((uint64_t)blockIdx.x * kPrecWarps + warp) * per;
+    if (start >= end_knot) return;  // warp-uniform; no CTA-wide barrier below
+    uint64_t gk = start;
+    const uint64_t end = min(gk + per, end_knot);
     // system owning global knot gk: last s with knot_prefix[s] <= gk (or the
     // one system passed by value)
     uint32_t lo = descs ? find_system(knot_prefix, nsys, gk, lane) : 0u;
     CT *s = sR[warp], *X = sX[warp];
     bool ok = true;
     while (gk < end) {
-        const uint32_t n = descs ? descs[lo].n : one.n, N = descs ? descs[lo].N : one.N;
-        const void *dS = descs ? descs[lo].S : one.S, *dP = descs ? descs[lo].P : one.P;
+        const SysDesc *d = descs ? descs + (sys ? sys[lo] : lo) : nullptr;
+        const uint32_t n = d ? d->n : one.n, N = d ? d->N : one.N;
+        const void *dS = d ? d->S : one.S, *dP = d ? d->P : one.P;
         const uint32_t k = (uint32_t)(descs ? gk - knot_prefix[lo] : gk);
         const uint32_t left = (uint32_t)min(end - gk, (uint64_t)(N - k));  // knots of this system in the range
         uint32_t cnt = left;
-        if (np_class(n) >= 0 && ((classes >> np_class(n)) & 1u)) {  // a class of this launch
+        if (np_class(n) >= 0) {
             cnt = min(left, n <= 8 ? 4u : (n <= 16 ? 2u : 1u));
             const TI *Sk = static_cast<const TI *>(dS) + (size_t)k * 3 * n * n + (size_t)n * n;
             TO *row = static_cast<TO *>(const_cast<void *>(dP)) + (size_t)k * (tri_layout ? 3 : 1) * n * n;
@@ -169,8 +171,7 @@ __global__ void __launch_bounds__(kPrecWarps * 32, sizeof(CT) == 4 ? 5 : 4)
         gk += cnt;
     }
     if (!__all_sync(0xffffffffu, ok)) {
-        gk = ((uint64_t)blockIdx.x * kPrecWarps + warp) * per;
-        invert_range_any<TI, TO, CT>(descs, nullptr, knot_prefix, nsys, gk, min(gk + per, total_knots), tri_layout, &one, s, X);
+        invert_range_any<TI, TO, CT>(descs, sys, knot_prefix, nsys, start, end, tri_layout, &one, s, X);
     }
 }
 
@@ -287,17 +288,19 @@ __device__ __forceinline__ bool invert_quads(const float *Sk, float *row, uint32
 // One launch per block-size class, so that an SM runs one class's code and a
 // narrow block does not pay for the registers of a wide one (all classes in one
 // kernel: 312 us where these take 190, 2048 systems of n in {6, 12, 14, 24}).
-// sys, knot_prefix: the class's systems and the knots before each; null: `one`.
+// sys, knot_prefix: the class's systems and the knots before each, whose knots are
+// [first_knot, end_knot); null: `one`.
 template <int NP>
 __global__ void __launch_bounds__(kQuadWarps * 32, NP <= 8 ? 12 : (NP <= 12 ? 9 : (NP <= 16 ? 8 : (NP <= 24 ? 6 : 4))))
     block_jacobi_quad_kernel(const SysDesc *__restrict__ descs, const uint32_t *__restrict__ sys,
-                             const uint64_t *__restrict__ knot_prefix, uint32_t nsys, uint64_t total_knots, uint32_t per,
-                             int tri_layout, const __grid_constant__ SysDesc one) {
+                             const uint64_t *__restrict__ knot_prefix, uint32_t nsys, uint64_t first_knot, uint64_t end_knot,
+                             uint32_t per, int tri_layout, const __grid_constant__ SysDesc one) {
     __shared__ __align__(16) float scratch[kQuadWarps][(quad_words<NP>() + 3) / 4 * 4];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint64_t gk = ((uint64_t)blockIdx.x * kQuadWarps + warp) * per;
-    if (gk >= total_knots) return;  // warp-uniform; no CTA-wide barrier below
-    const uint64_t end = min(gk + per, total_knots);
+    const uint64_t start = first_knot + ((uint64_t)blockIdx.x * kQuadWarps + warp) * per;
+    if (start >= end_knot) return;  // warp-uniform; no CTA-wide barrier below
+    uint64_t gk = start;
+    const uint64_t end = min(gk + per, end_knot);
     uint32_t lo = sys ? find_system(knot_prefix, nsys, gk, lane) : 0u;
     bool ok = true;
     while (gk < end) {
@@ -317,9 +320,8 @@ __global__ void __launch_bounds__(kQuadWarps * 32, NP <= 8 ? 12 : (NP <= 12 ? 9 
     }
     if (!__all_sync(0xffffffffu, ok)) {
         static_assert(quad_words<NP>() >= 32 + NP * NP, "scratch of the other inverse");
-        gk = ((uint64_t)blockIdx.x * kQuadWarps + warp) * per;
-        invert_range_any<float, float, float>(sys ? descs : nullptr, sys, knot_prefix, nsys, gk, min(gk + per, total_knots),
-                                                tri_layout, &one, scratch[warp], scratch[warp] + 32);
+        invert_range_any<float, float, float>(sys ? descs : nullptr, sys, knot_prefix, nsys, start, end, tri_layout, &one,
+                                              scratch[warp], scratch[warp] + 32);
     }
 }
 
@@ -337,8 +339,7 @@ cudaError_t launch_block_jacobi(int kind, const SysDesc *d_descs, const uint64_t
     SysDesc o;
     if (one) o = *one;
     else memset(&o, 0, sizeof(o));
-    uint32_t classes = 0x1f;  // left to the kernel with one row a lane
-    uint64_t rest = total_knots;
+    bool quads[5] = {};  // classes of the kernel with four rows a lane
     if (kind == 0) {
         auto quad = [&](auto np) {
             constexpr int NP = decltype(np)::value, c = np_class(NP);
@@ -346,35 +347,57 @@ cudaError_t launch_block_jacobi(int kind, const SysDesc *d_descs, const uint64_t
             if (knots < kQuadFrom) return;
             const uint32_t *sys = one ? nullptr : cls->sys + cls->first[c];
             const uint64_t *prefix = one ? nullptr : cls->prefix + cls->first[c];
+            const uint64_t first = one ? 0 : cls->base[c];
             const uint32_t per = GjQuad<NP>::BLOCKS * (knots >= (uint64_t)GjQuad<NP>::BLOCKS * 4096 ? 2 : 1);
             const uint64_t warps = (knots + per - 1) / per;
             block_jacobi_quad_kernel<NP><<<(unsigned)((warps + kQuadWarps - 1) / kQuadWarps), kQuadWarps * 32, 0, stream>>>(
-                d_descs, sys, prefix, one ? 1u : cls->count[c], knots, per, tri_layout, o);
-            classes &= ~(1u << c);
-            rest -= knots;
+                d_descs, sys, prefix, one ? 1u : cls->count[c], first, first + knots, per, tri_layout, o);
+            quads[c] = true;
         };
         quad(std::integral_constant<int, 24>());
         quad(std::integral_constant<int, 32>());
         quad(std::integral_constant<int, 16>());
         quad(std::integral_constant<int, 12>());
         quad(std::integral_constant<int, 8>());
-        if (rest == 0) return cudaGetLastError();
     }
-    // knots a warp: side by side while the GPU has warps to spare, then several, as
-    // many as a warp inverts at once for a single system
-    const uint32_t most = d_descs ? 4u : (o.n <= 8 ? 4u : (o.n <= 16 ? 2u : 1u));
-    const uint32_t per = rest < 8192 ? 1u : (rest < 32768 ? (most < 2 ? most : 2u) : most);
-    const uint64_t warps = (total_knots + per - 1) / per;
-    const dim3 grid((unsigned)((warps + kPrecWarps - 1) / kPrecWarps)), block(kPrecWarps * 32);
-    if (kind == 1)
-        block_jacobi_kernel<double, double, double><<<grid, block, 0, stream>>>(
-            d_descs, d_prefix, nsys, total_knots, per, tri_layout, classes, o);
-    else if (kind == 2)
-        block_jacobi_kernel<double, float, double><<<grid, block, 0, stream>>>(
-            d_descs, d_prefix, nsys, total_knots, per, tri_layout, classes, o);
-    else
-        block_jacobi_kernel<float, float, float><<<grid, block, 0, stream>>>(
-            d_descs, d_prefix, nsys, total_knots, per, tri_layout, classes, o);
+    // one row a lane for knots [first, first + knots) of the order of `sys`
+    auto rest = [&](const uint32_t *sys, const uint64_t *prefix, uint32_t count, uint64_t first, uint64_t knots) {
+        // knots a warp: side by side while the GPU has warps to spare, then several, as
+        // many as a warp inverts at once for a single system
+        const uint32_t most = d_descs ? 4u : (o.n <= 8 ? 4u : (o.n <= 16 ? 2u : 1u));
+        const uint32_t per = knots < 8192 ? 1u : (knots < 32768 ? (most < 2 ? most : 2u) : most);
+        const uint64_t warps = (knots + per - 1) / per;
+        const dim3 grid((unsigned)((warps + kPrecWarps - 1) / kPrecWarps)), block(kPrecWarps * 32);
+        if (kind == 1)
+            block_jacobi_kernel<double, double, double><<<grid, block, 0, stream>>>(d_descs, sys, prefix, count, first,
+                                                                                    first + knots, per, tri_layout, o);
+        else if (kind == 2)
+            block_jacobi_kernel<double, float, double><<<grid, block, 0, stream>>>(d_descs, sys, prefix, count, first,
+                                                                                   first + knots, per, tri_layout, o);
+        else
+            block_jacobi_kernel<float, float, float><<<grid, block, 0, stream>>>(d_descs, sys, prefix, count, first,
+                                                                                 first + knots, per, tri_layout, o);
+    };
+    bool any = false;
+    for (bool q : quads) any |= q;
+    if (!any) {
+        rest(nullptr, d_prefix, nsys, 0, total_knots);
+    } else if (!one) {
+        // runs of neighbouring classes that are left: their knots only (with one launch
+        // over all knots, most of whose warps found nothing to do, 1000 systems of n=6
+        // and 10 of n=24, 100 knots each, took 74 us; now 32)
+        for (int c = 0; c < 5;) {
+            int e = c;
+            uint32_t count = 0;
+            uint64_t knots = 0;
+            for (; e < 5 && !quads[e]; ++e) {
+                count += cls->count[e];
+                knots += cls->knots[e];
+            }
+            if (knots) rest(cls->sys + cls->first[c], cls->prefix + cls->first[c], count, cls->base[c], knots);
+            c = e + 1;
+        }
+    }
     return cudaGetLastError();
 }
 
