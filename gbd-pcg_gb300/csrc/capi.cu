@@ -325,17 +325,23 @@ uint32_t ctas_per_sm(const Shape &s) {
 // CTAs an SM) 274 / 217; n=24 N=16 304 / 365, N=10 (two) 238 / 175; n=12 N=42
 // 285 / 324, N=32 (two) 263 / 170; n=8 N=96 347 / 429, N=64 (two) 257 / 205;
 // n=6 N=128 358 / 502, N=85 (two) 271 / 239; n=24 N=64, C 2 against 4,
-// 516 / 1046 for 600.  When all of a plan's systems run at once (`one_wave`)
-// every SM holds at most one CTA either way and tensor memory's shorter pass
-// wins everywhere: 152 systems of n=14 N=11 33 / 44, n=6 N=64 42 / 61.
+// 516 / 1046 for 600.
 // Refinement: 256 x n=24 N=256 with C 8 against 16, 91 against 181 ms; 64 x
 // n=24 N=64 5.6 / 8.7; 200 x n=14 N=100 16.7 / 19.3; 256 x n=8 N=32 (three
 // split CTAs an SM) 4.7 / 3.6.
-bool tmem_pays(const Shape &t, const Shape &s, bool one_wave) {
-    return t.C * ctas_per_sm(s) <= s.C || (one_wave && t.C <= s.C);
-}
+bool tmem_pays(const Shape &t, const Shape &s) { return t.C * ctas_per_sm(s) <= s.C; }
 
-//
+// When all of a plan's systems run at once (`one_wave`) every SM holds at most one
+// of its CTAs either way, and tensor memory's shorter pass wins: 152 systems of
+// n=14 N=11 33 / 44 us, n=6 N=64 42 / 61.  That is for a plan that has the GPU to
+// itself: several such plans at once on streams of their own fill the SMs with
+// split rows' smaller CTAs (152 of n=14 N=27, us a plan on 1 / 2 / 4 streams: tensor
+// memory 40 / 35 / 35, split 52 / 29 / 26), and their caller pins split rows.
+// Only at the cluster and CTA size that the split rows have: both storages then
+// give the same bits, so lambda does not depend on what else is in the plan (or
+// on the piece of a host pipeline a system is in).
+bool tmem_alone(const Shape &t, const Shape &s) { return t.C == s.C && t.threads == s.threads; }
+
 // c_pref > 1 (lone systems, cluster size not pinned): clusters from c_pref up
 // are tried first, then the smallest that fits.  `lone`: a single system
 // solved by itself.  For such a system with a cbtd Phi^-1 that no on-chip
@@ -423,14 +429,18 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
             // (a lone FP32 system has tried tensor memory first)
             if (cfg.storage == GBDPCG_STORAGE_AUTO && !ptri && (refine || (!lone && !f64))) {
                 Shape t;
-                if (fit(Pref{4, 2}, from, &t) && tmem_pays(t, s, one_wave && !refine)) {
-                    // three CTAs at most three quarters full: four, with shorter
-                    // passes (n=24 N=72: 45 against 52 us for one system, 911
-                    // against 857 for 600 of them)
+                const bool fits = fit(Pref{4, 2}, from, &t);
+                if (fits && tmem_pays(t, s)) {
+                    // three CTAs at most three quarters full: four, whose passes are
+                    // shorter and whose sums are the lone call's (n=24 N=72: 45 against
+                    // 52 us for one system; 600 of them 911 against 857, and 1046 with
+                    // split rows)
                     Shape t4;
                     if (!refine && t.C == 3 && t.K * n * 4 <= (uint32_t)t.vi->max_threads * 2 * 3 && s.C >= 4 &&
                         fit(Pref{4, 2}, 4, &t4) && t4.C == 4)
                         t = t4;
+                    s = t;
+                } else if (fits && one_wave && !refine && tmem_alone(t, s)) {
                     s = t;
                 }
             }
