@@ -97,9 +97,12 @@ __device__ __forceinline__ void acc_madd(A &v, T a, T b) {
 // float(a / b) of two doubles without the FP64 pipe (a double division is about
 // ten dependent FP64 instructions): the operands' mantissas as float pairs, one
 // float division, one correction with the remainder (as for f2acc below), and
-// the exponents put back.  Within 2^-45 of the quotient before its rounding to
-// float; zeros, subnormals, non-finite operands and quotients near or past the
-// range of float go through the double division.
+// the exponents put back.  The sum of quotient and correction is within 2^-45 of
+// a / b, so rounding it to float is rounding a / b, unless what that rounding
+// drops is within 2^-43 of half an ulp, or the result is a power of two, below
+// which ulps are shorter.  Those quotients (three in a million), zeros, subnormals,
+// non-finite operands and quotients near or past the range of float go through
+// the double division.
 __device__ __forceinline__ float ratio_f32(double a, double b) {
     const uint32_t ah = (uint32_t)__double2hiint(a), bh = (uint32_t)__double2hiint(b);
     const uint32_t al = (uint32_t)__double2loint(a), bl = (uint32_t)__double2loint(b);
@@ -114,7 +117,11 @@ __device__ __forceinline__ float ratio_f32(double a, double b) {
     float r = __fmaf_rn(-q, b0, a0);  // exact
     r = __fadd_rn(r, a1);
     r = __fmaf_rn(-q, b1, r);
-    const float v = __fadd_rn(q, __fdiv_rn(r, b0));
+    const float c = __fdiv_rn(r, b0), v = __fadd_rn(q, c);
+    const float dropped = __fsub_rn(c, __fsub_rn(v, q));  // exact
+    const uint32_t vb = __float_as_uint(v);
+    const float half = __uint_as_float((vb & 0x7f800000u) - (24u << 23));
+    if (fabsf(__fsub_rn(fabsf(dropped), half)) < 1.1368683772161603e-13f || (vb & 0x7fffffu) == 0u) return (float)(a / b);
     // 2^k with the quotient's sign
     return __fmul_rn(v, __uint_as_float(((ah ^ bh) & 0x80000000u) | ((uint32_t)(k + 127) << 23)));
 }
