@@ -483,7 +483,7 @@ struct gbdpcg_handle_s {
     // the kernel writes, so that reading it after the stream has ended takes no
     // copy (49.3 -> 43.5 us for a call of n=14 N=32).  A solve that nobody waits for
     // leaves its result in device memory (`ws`): the kernel ends without a write
-    // over the link.
+    // over the link.  (Null where no pinned memory was to be had: `ws` for all.)
     SysResult *result = nullptr;
     SysResult *d_last = nullptr;
     cudaStream_t last_stream = nullptr;
@@ -659,8 +659,8 @@ bool grid_pays(const Shape &sh, const SysDesc &d, const gbdpcg_config &cfg, bool
 }
 
 // Solves `d` on the whole GPU; *done stays false where the launch does not apply
-// (a shape it does not hold, a stream that is being captured, CTAs that cannot
-// all be resident): the caller then takes another kernel.
+// (a shape it does not hold, a stream that is being captured, no memory for the
+// mailboxes, CTAs that cannot all be resident): the caller then takes another kernel.
 int solve_grid(gbdpcg_handle_s *h, bool f64, const SysDesc &d, uint32_t layout, SysResult *d_res, cudaStream_t stream,
                bool *done) {
     *done = false;
@@ -694,9 +694,14 @@ int solve_grid(gbdpcg_handle_s *h, bool f64, const SysDesc &d, uint32_t layout, 
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = h->device;
-            GB_CUDA(cudaMemPoolCreate(&h->pool, &props));
             uint64_t keep = UINT64_MAX;
-            GB_CUDA(cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+            if (cudaMemPoolCreate(&h->pool, &props) != cudaSuccess ||
+                cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+                cudaGetLastError();  // (the next call tries again)
+                if (h->pool) cudaMemPoolDestroy(h->pool);
+                h->pool = nullptr;
+                return GBDPCG_SUCCESS;
+            }
         }
     }
     GB_CUDA(allow_dynamic_smem(gv->func, smem));
@@ -730,7 +735,7 @@ int solve_grid(gbdpcg_handle_s *h, bool f64, const SysDesc &d, uint32_t layout, 
 // One system, device pointers; result left in h->d_last.
 int solve_one(gbdpcg_handle_s *h, bool f64, const SysDesc &d0, const gbdpcg_config &cfg,
               uint32_t layout, cudaStream_t stream, bool waits, bool refine = false) {
-    SysResult *d_res = waits ? h->result : h->ws.as<SysResult>();
+    SysResult *d_res = waits && h->result ? h->result : h->ws.as<SysResult>();
     int rc;
     SysDesc d = d0;
     d.result = 0;
@@ -1035,8 +1040,8 @@ int gbdpcg_create(gbdpcg_handle_t *handle, int device) {
     if (rc) return rc;
     if (cudaHostAlloc(reinterpret_cast<void **>(&h->result), sizeof(SysResult), cudaHostAllocMapped | cudaHostAllocPortable) !=
         cudaSuccess) {
+        cudaGetLastError();
         h->result = nullptr;
-        return fail(GBDPCG_ERR_NO_MEMORY, "cudaHostAlloc of the result");
     }
     *handle = h.release();
     return GBDPCG_SUCCESS;
@@ -1084,7 +1089,7 @@ int gbdpcg_solve_dev_f64(gbdpcg_handle_t h, const double *d_S, const double *d_P
 int gbdpcg_last_result(gbdpcg_handle_t h, gbdpcg_result *result) {
     if (!h || !result || !h->d_last) return fail(GBDPCG_ERR_INVALID_ARGUMENT, "no result");
     HandleScope scope(h->device);
-    if (h->d_last == h->result) {
+    if (h->result && h->d_last == h->result) {
         GB_CUDA(cudaStreamSynchronize(h->last_stream));
         to_public(*h->result, result);
         return GBDPCG_SUCCESS;
