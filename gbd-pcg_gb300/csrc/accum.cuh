@@ -107,7 +107,6 @@ __device__ __forceinline__ float ratio_f32(double a, double b) {
     const uint32_t ah = (uint32_t)__double2hiint(a), bh = (uint32_t)__double2hiint(b);
     const uint32_t al = (uint32_t)__double2loint(a), bl = (uint32_t)__double2loint(b);
     const int ea = (int)((ah >> 20) & 0x7ffu), eb = (int)((bh >> 20) & 0x7ffu), k = ea - eb;
-    if (ea == 0 || eb == 0 || ea == 0x7ff || eb == 0x7ff || k > 120 || k < -120) return (float)(a / b);
     // mantissa in [1, 2): the leading 23 bits as a float, the other 29 scaled by 2^-52
     const float a0 = __uint_as_float(0x3f800000u | ((ah & 0xfffffu) << 3) | (al >> 29));
     const float b0 = __uint_as_float(0x3f800000u | ((bh & 0xfffffu) << 3) | (bl >> 29));
@@ -121,7 +120,9 @@ __device__ __forceinline__ float ratio_f32(double a, double b) {
     const float dropped = __fsub_rn(c, __fsub_rn(v, q));  // exact
     const uint32_t vb = __float_as_uint(v);
     const float half = __uint_as_float((vb & 0x7f800000u) - (24u << 23));
-    if (fabsf(__fsub_rn(fabsf(dropped), half)) < 1.1368683772161603e-13f || (vb & 0x7fffffu) == 0u) return (float)(a / b);
+    const bool range = (uint32_t)(ea - 1) < 0x7feu && (uint32_t)(eb - 1) < 0x7feu && (uint32_t)(k + 120) <= 240u;
+    const bool safe = fabsf(__fsub_rn(fabsf(dropped), half)) >= 1.1368683772161603e-13f && (vb & 0x7fffffu) != 0u;
+    if (!(range && safe)) return (float)(a / b);
     // 2^k with the quotient's sign
     return __fmul_rn(v, __uint_as_float(((ah ^ bh) & 0x80000000u) | ((uint32_t)(k + 127) << 23)));
 }
