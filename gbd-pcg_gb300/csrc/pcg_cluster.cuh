@@ -1488,16 +1488,21 @@ __global__ void __launch_bounds__((RegBudget<T, A, NP, PTRI, ST, RPT>::max_threa
                     }
                     if constexpr (kOneWarpSums<A>) {
                         // the first half's CTA barrier completes this CTA's z rows in the window
+                        // FP64 rows: the product after the reduction.  Before it the other warps'
+                        // FP64 instructions queue in front of the summing warps' additions, for
+                        // which every CTA waits (200 systems of n=28 N=40 5003 -> 3753 us, 300 of
+                        // n=14 N=64 1753 -> 1547).
+                        constexpr bool kAfter = sizeof(T) == 8;
                         onewarp_send<A, 2>(v2, slots, wscr, 1, tx, C, rank, halo_in);
                         const bool halo_rows = C > 1 && __any_sync(0xffffffffu, first_knot || last_knot);
-                        if (!halo_rows) matS_rows(w);
+                        if (!kAfter && !halo_rows) matS_rows(w);
                         const ReduceOut *o = onewarp_finish<A, 2>(
                             v2, slots, 1, tx, C,
                             [&](int q, A s, ReduceOut *out) { onewarp_beta<T>(q, s, eta, tol, thr, out, tid & 31); });
                         beta_h = *reinterpret_cast<const T *>(&o->ratio);
                         code1 |= o->code[0] & kNotFinite;
                         code2 = o->code[relres ? 1 : 0];
-                        if (halo_rows) matS_rows(w);
+                        if (kAfter || halo_rows) matS_rows(w);
                     } else if (C > 1) {
                         // its CTA barrier also completes this CTA's z rows in the window
                         cluster_allreduce_tx_send<A, 2>(v2, slots, wscr, 1, tx, C, rank, halo_in);
