@@ -131,6 +131,21 @@ def whole_job_rate(job_systems, steps, seconds):
     return job_systems * steps / seconds
 
 
+# Sections that explain the result: some 22 KB, too long for one line of a log that
+# keeps only its end (the result could not be read back from it).
+DETAIL = ("single_system", "single_system_n128", "adjoint", "precision", "around_solve", "block_jacobi", "timeline")
+
+
+def split_line(line):
+    """The result line, a few KB, and what explains it (printed on stderr)."""
+    result = {k: v for k, v in line.items() if k not in DETAIL}
+    detail = {k: line[k] for k in DETAIL if k in line}
+    if "launch_shapes" in result.get("config", {}):
+        result["config"] = dict(result["config"])
+        detail["launch_shapes"] = result["config"].pop("launch_shapes")
+    return result, detail
+
+
 def algorithmic_bytes(descs, iters, s=4):
     it = np.asarray(iters, np.float64)
     n = np.array([d[0] for d in descs], np.float64)
@@ -1095,7 +1110,10 @@ def main():
             line["roofline"]["latency"] = {
                 k: {"floor_us_per_iter": v["floor_us_per_iter"], "achieved_us_per_iter": v["achieved_us_per_iter"],
                     "frac": v["frac"], "shape": v["shape"]} for k, v in lat.items()}
-    print(json.dumps(line), flush=True)
+    result, detail = split_line(line)
+    if detail:
+        print(json.dumps({"detail": detail}), file=sys.stderr, flush=True)
+    print(json.dumps(result), flush=True)
     plan.close()
     h.close()
     if world > 1:
