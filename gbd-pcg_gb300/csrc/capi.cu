@@ -242,7 +242,12 @@ std::vector<Pref> storage_prefs(bool f64, bool ptri, uint32_t storage) {
 // single-reduction, refinement and streamed kernels have no such row).  Two rows
 // a thread share every vector load and fit tensor memory: 600 systems of n in {4,
 // 7, 13, 14, 21}, 10 to 100 knots, 666 us with one row a thread for the odd ones,
-// 377 so.
+// 377 so.  Short systems of small odd blocks are slower so between the plans that
+// tensor memory serves and those that fill every SM: n=3 N=16, us, one row / two, 100
+// systems 34 / 28, 300 34 / 42, 1000 38 / 48; n=7 N=16 36 / 28, 36 / 40, 73 / 49.  A
+// rule by the size alone, which keeps a system's bits the same in every batch, gains
+// at one count what it loses at another (600 mixed ones 367 -> 400 us); a caller with
+// such a batch pins registers.
 bool rows_pair(uint32_t n, int st, int rpt, int alg) {
     return n % (uint32_t)rpt == 0 || ((alg == 0 || alg == 3) && !streamed(st));
 }
@@ -380,9 +385,8 @@ int choose_shape(Registry *reg, bool f64, uint32_t n, uint32_t N, uint32_t layou
     const uint32_t first_lo = (cfg.cluster_size == 0 && c_pref > 1) ? c_pref : 1;
     std::vector<Pref> prefs = storage_prefs(f64 && !refine, ptri, cfg.storage);
     // A lone FP32 system takes tensor-memory rows first where they fit: its
-    // CTAs have their SMs to themselves anyway (the exclusive tensor-memory
-    // allocation is what keeps that storage out of AUTO for batches), and its
-    // iteration is the shortest there (n = 14, N = 32: 1.1-1.3 us against
+    // CTAs have their SMs to themselves anyway, and its iteration is the
+    // shortest there (n = 14, N = 32: 1.1-1.3 us against
     // 1.4-1.6 us with S in registers and Phi^-1 in shared memory).
     if (lone && cfg.storage == GBDPCG_STORAGE_AUTO && !f64 && !refine && !ptri)
         prefs.insert(prefs.begin(), Pref{4, 2});
@@ -652,6 +656,12 @@ int max_active_clusters(const Shape &sh, size_t smem, int *out) {
 // n=14 N=440 674 / 573, n=24 N=200 654 / 416, cbtd n=24 N=100 650 / 500.  On
 // chip / whole GPU: FP32 n=14 N=1100 92 / 186, cbtd N=512 163 / 191; FP64 n=14
 // N=256 298 / 382, cbtd N=128 339 / 406.
+// That is for a call that has the GPU to itself.  Solves on several streams at once
+// share it: up to four whole-GPU kernels are still the faster (FP32 n=14 N=1500, four
+// streams, us a solve 140 / 76; FP64 n=14 N=1000 209 / 170; not FP64 n=6 N=8000 283 /
+// 331), eight are for large FP32 blocks (n=14 N=8192 472 / 189), not for FP64 or small
+// ones (FP64 n=14 N=1000 125 / 167, n=6 N=8000 170 / 330; FP32 n=6 N=5000 50 / 69):
+// their caller pins streamed rows or a cluster size.
 bool grid_pays(const Shape &sh, const SysDesc &d, const gbdpcg_config &cfg, bool refine) {
     return !refine && cfg.algorithm == GBDPCG_ALGO_AUTO && cfg.storage == GBDPCG_STORAGE_AUTO && !cfg.cluster_size &&
            !cfg.max_threads && cfg.dot_precision == GBDPCG_DOT_NATIVE && !(d.flags & SYS_ADJOINT) &&
@@ -1202,8 +1212,11 @@ static int solve_host(bool f64, const void *S, const void *P, const void *g, voi
     // same bits either way.
     const char *stage_env = getenv("GBDPCG_HOST_STAGING");
     bool direct = h->reg->host_direct && !(stage_env && stage_env[0] == '1');
-    // (no system below a MiB of S goes to a kernel that reads its rows in every
-    // pass; those that do are staged, or every pass would read host memory)
+    // Systems of the whole-GPU kernel, which reads Phi^-1 (and S past the registers)
+    // in every pass, are staged from a MiB of S on, so that a pass reads device
+    // memory.  Below that they are as fast in place: cbtd n=2 N=20000 491 us, staged
+    // 532; n=3 N=8000 587 / 549; n=4 N=4500 312 / 354; FP64 n=2 N=8000 777 / 763.
+    // (Pinned streamed rows and the plain algorithm read host arrays in place.)
     if (direct && mat >= ((size_t)1 << 20)) {
         Shape sh;
         SysDesc d = make_desc(S, P, g, l, l, n, N, c, build_layout, 0);

@@ -182,7 +182,7 @@ __device__ __forceinline__ void gram_tile(const T *Mt, uint32_t ldt, const T *dv
 //
 // What bounds it: instruction issue and the shared-memory pipe (n=24, m=12: 5930
 // instructions a knot with one element an access, one row an FMA and a select an
-// element of the inverse; now 4200, the pipe 71% busy).  Measured, us, before
+// element of the inverse; now 4035, the pipe 84% busy).  Measured, us, before
 // and now, N=65536 FP32: n=24 m=12 212 -> 183, with Phi^-1 382 -> 322; n=14 m=7
 // 114 -> 102, 198 -> 140; n=6 m=3 with Phi^-1 96 -> 56.  FP64 is bound by the FP64
 // pipe (n=14 m=7 N=30000 with Phi^-1 1365 -> 862), so it takes 16-byte accesses only

@@ -37,8 +37,8 @@
 // What bounds it: two exchanges an iteration (stores to L2, a poll from it, the
 // CTA-wide stages: about 2.3 us each), then the products (n=14 N=8192: 1.3 us
 // with S in registers, 2.7 from the L1).  One system of n=14 N=8192 FP32, 39
-// passes: 2150 us with streamed rows on 16 SMs, 240 us here, 299 with S from
-// the L1; N=20000 5916 against 445.  The rule with both sides measured is
+// passes, device time: 2150 us with streamed rows on 16 SMs, 240 us here, 299 with S
+// from the L1; N=20000 5916 against 445.  The rule with both sides measured is
 // grid_pays in capi.cu.
 #pragma once
 #include "pcg_cluster.cuh"

@@ -23,7 +23,7 @@
 //
 // Measured, FP32, us, one block a warp with a scaled pivot row / one row a lane /
 // four: 2048 systems of 16 to 128 knots, n=14 302 / 143 / 108, n=6 173 / 57 / 34,
-// n in {6, 12, 14, 24} 317 / 225 / 190; 1024 of n=24 269 / 250 / 181; 512 of n=32
+// n in {6, 12, 14, 24} 317 / 225 / 182; 1024 of n=24 269 / 250 / 181; 512 of n=32
 // 223 / 287 / 181.  What bounds four rows a lane is the fetch of its long
 // straight-line code by two or three warps a scheduler (n=24: 990 instructions a
 // block, issued at 37%).  TI: element type of S, TO: of Phi^-1, CT: arithmetic (double S
@@ -287,7 +287,7 @@ __device__ __forceinline__ bool invert_quads(const float *Sk, float *row, uint32
 
 // One launch per block-size class, so that an SM runs one class's code and a
 // narrow block does not pay for the registers of a wide one (all classes in one
-// kernel: 312 us where these take 190, 2048 systems of n in {6, 12, 14, 24}).
+// kernel: 312 us where these take 182, 2048 systems of n in {6, 12, 14, 24}).
 // sys, knot_prefix: the class's systems and the knots before each, whose knots are
 // [first_knot, end_knot); null: `one`.
 template <int NP>

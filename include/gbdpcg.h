@@ -203,7 +203,10 @@ GBDPCG_API int gbdpcg_solve_f64(const double *S, const double *Pinv, const doubl
  * d_r, d_p, d_v_temp, d_eta_new_temp, config) (include/interface.cuh:94-146);
  * the cluster solver keeps r and p on chip, so no scratch is passed.  If
  * `result` is non-NULL the call waits for the stream and fills it; else the
- * result stays on the device (gbdpcg_last_result). */
+ * result stays on the device (gbdpcg_last_result).  Solves may be in flight on
+ * several streams; those of one handle that take the plain algorithm run one
+ * after another (captured ones: in the order of their replays, which the caller
+ * keeps apart). */
 GBDPCG_API int gbdpcg_solve_dev_f32(gbdpcg_handle_t h, const float *d_S, const float *d_Pinv,
                          uint32_t pinv_layout, const float *d_gamma, float *d_lambda, uint32_t n,
                          uint32_t N, const gbdpcg_config *cfg, gbdpcg_result *result,
@@ -232,7 +235,8 @@ GBDPCG_API int gbdpcg_last_result(gbdpcg_handle_t h, gbdpcg_result *result);
  * GBDPCG_NOALLOC_MAX_ELEMS and N <= GBDPCG_NOALLOC_MAX_KNOTS, else
  * GBDPCG_ERR_UNSUPPORTED.  The config is checked like the handle entry
  * points' configs.  No handle, no cudaMalloc/cudaFree.  Calls share the
- * array: calls that overlap on the GPU race.  If `result` is non-NULL the
+ * array: calls that overlap on the GPU race and can wait for one another without
+ * end, so the caller orders them.  If `result` is non-NULL the
  * call waits for the stream and fills it. */
 #define GBDPCG_NOALLOC_MAX_ELEMS 131072
 #define GBDPCG_NOALLOC_MAX_KNOTS 4096
