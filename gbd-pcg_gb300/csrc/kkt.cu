@@ -343,16 +343,21 @@ __global__ void __launch_bounds__(W * 32, schur_ctas<T, NP, PINV>())
 }
 
 // s + sum_j col[j] w[j], j ascending, VW elements an access (n a multiple of VW,
-// both addresses aligned to it), U accesses an iteration.
+// both addresses aligned to it), U accesses an iteration (0: as the compiler has it).
 template <typename T, int VW, int U>
 __device__ __forceinline__ T col_dot(const T *col, const T *w, uint32_t n, T s) {
-#pragma unroll U
-    for (uint32_t j = 0; j < n; j += VW) {
+    auto add = [&](uint32_t j) {
         T a[VW], b[VW];
         load_vec<T, VW>(col + j, a);
         load_vec<T, VW>(w + j, b);
 #pragma unroll
         for (int u = 0; u < VW; ++u) s += a[u] * b[u];
+    };
+    if constexpr (U == 0) {
+        for (uint32_t j = 0; j < n; j += VW) add(j);
+    } else {
+#pragma unroll U
+        for (uint32_t j = 0; j < n; j += VW) add(j);
     }
     return s;
 }
@@ -364,16 +369,17 @@ __device__ __forceinline__ T col_dot(const T *col, const T *w, uint32_t n, T s) 
 // L1 of an SM's 64 warps (n=24 m=12: 55 us against 50; n=24 m=8 46 / 44, n=16 m=8
 // 31.3 / 32.0).  A lane reads its own
 // contiguous column with accesses of 16 or 8 bytes where n and the addresses allow,
-// U an iteration: one where every lane has a column to read, four where the lanes
-// beyond the block's columns wait (TWO) or an access is 4 bytes.
+// U an iteration: one for 16-byte accesses in one pass and for FP64 in one pass, four
+// for FP64 in two, as the compiler has it for the rest (n=13 m=6 N=60000: 21.7 us so,
+// 23.6 with four).
 //
 // What bounds it: HBM and, for short columns, the L1 requests (a column is 24 to
 // 128 bytes).  Measured, us, before (one pass for A_k, one for B_k, one element an
 // access unless n is a multiple of 4) and now, one problem again and again (n=14: its
 // 70 MB lie in the L2) / eight problems in turn (n=6: in the L2 still): n=14
-// m=7 N=60000 27.6 -> 19.7 / 31.6 -> 25.7, n=6 m=3 21.3 -> 9.8 / 27.0 -> 9.8, n=12
-// m=6 19.2 -> 14.9 / 27.4 -> 18.8, n=13 m=6 25.2 -> 23.7 / 30.3 -> 27.4, n=22 m=11
-// 56.1 -> 45.7 / 55.8 -> 45.1; FP64 n=14 m=7 N=30000 81.8 -> 60.4 / 82.4 -> 62.0.
+// m=7 N=60000 27.6 -> 21.7 / 31.6 -> 25.2, n=6 m=3 21.3 -> 9.8 / 27.0 -> 9.8, n=12
+// m=6 19.2 -> 14.9 / 27.4 -> 18.8, n=13 m=6 25.2 -> 21.7 / 30.3 -> 25.0, n=22 m=11
+// 56.1 -> 42.6 / 55.8 -> 42.3; FP64 n=14 m=7 N=30000 81.8 -> 60.4 / 82.4 -> 62.0.
 // n=24 m=12 (47.5 -> 44.2) and FP64 of 25 columns or more, bound by its pipe, are
 // as they were.
 template <typename T, int GL, int VW, bool TWO, int kKktWarps>
@@ -382,7 +388,7 @@ __global__ void __launch_bounds__(kKktWarps * 32)
                        const T *__restrict__ Rd, const T *__restrict__ q, const T *__restrict__ r,
                        const T *__restrict__ lambda, uint32_t n, uint32_t m, uint32_t N, T *__restrict__ x,
                        T *__restrict__ u) {
-    constexpr int U = TWO || (sizeof(T) == 4 && VW == 1) ? 4 : 1;
+    constexpr int U = sizeof(T) == 8 ? (TWO ? 4 : 1) : (VW == 4 && !TWO ? 1 : 0);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t k = (blockIdx.x * kKktWarps + (threadIdx.x >> 5)) * (32 / GL) + lane / GL;
     if (k > N) return;  // knots 0..N (x) and 0..N-1 (u)
