@@ -377,10 +377,10 @@ __device__ __forceinline__ T col_dot(const T *col, const T *w, uint32_t n, T s) 
 // 128 bytes).  Measured, us, before (one pass for A_k, one for B_k, one element an
 // access unless n is a multiple of 4) and now, one problem again and again (n=14: its
 // 70 MB lie in the L2) / eight problems in turn (n=6: in the L2 still): n=14
-// m=7 N=60000 27.6 -> 21.7 / 31.6 -> 25.2, n=6 m=3 21.3 -> 9.8 / 27.0 -> 9.8, n=12
+// m=7 N=60000 27.6 -> 21.7 / 31.6 -> 25.2, n=6 m=3 21.3 -> 10.2 / 27.0 -> 12.5, n=12
 // m=6 19.2 -> 14.9 / 27.4 -> 18.8, n=13 m=6 25.2 -> 21.7 / 30.3 -> 25.0, n=22 m=11
 // 56.1 -> 42.6 / 55.8 -> 42.3; FP64 n=14 m=7 N=30000 81.8 -> 60.4 / 82.4 -> 62.0.
-// n=24 m=12 (47.5 -> 44.2) and FP64 of 25 columns or more, bound by its pipe, are
+// n=24 m=12 (47.5) and FP64 of 25 columns or more, bound by its pipe, are
 // as they were.
 template <typename T, int GL, int VW, bool TWO, int kKktWarps>
 __global__ void __launch_bounds__(kKktWarps * 32)
